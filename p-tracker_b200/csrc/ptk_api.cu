@@ -703,13 +703,12 @@ int enqueue_subpixel(ptk_ctx* c, int method, cudaStream_t s) {
     CK(cudaMemsetAsync(lp.redo_count, 0, sizeof(int), s));
     launch_subpix_lm(c->g, frame(c, c->cur_slot), lp, s);
     if (lp.redo_list) {  // those grains: the reference's Powell from their pixel-stage state
-      launch_subpix_powell(c->g, frame(c, c->cur_slot), frame(c, c->ref_slot), subpix_params(c), c->max_P, c->max_R,
-                           lp.redo_list, s, lp.redo_count);
+      launch_subpix_powell(c->g, frame(c, c->cur_slot), subpix_params(c), c->max_P, c->max_R, c->num_sms, lp.redo_list,
+                           s, lp.redo_count);
       c->launches += 1;
     }
   } else if (method == PTK_SUBPIX_POWELL) {
-    launch_subpix_powell(c->g, frame(c, c->cur_slot), frame(c, c->ref_slot), subpix_params(c), c->max_P, c->max_R,
-                         c->d_order, s);
+    launch_subpix_powell(c->g, frame(c, c->cur_slot), subpix_params(c), c->max_P, c->max_R, c->num_sms, c->d_order, s);
   } else {
     return fail(c, PTK_ERR_ARG, "unknown subpixel method");
   }
@@ -1564,7 +1563,7 @@ int ptk_track_frame(ptk_ctx* c, int num_image) {
       SearchGeom sg;
       if ((rc = search_geometry(c, l, &sg))) return rc;
     }
-    prepare_subpix(c->max_P, c->max_R);
+    prepare_subpix(c->n, c->max_P, c->max_R, c->num_sms);
     const int64_t before = c->launches;
     CK(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeRelaxed));
     rc = enqueue_frame(c, pre, swap, c->cap_stream);

@@ -4,10 +4,11 @@
 // The objective (objective_exact) follows the reference's FP64 operations
 // (src/p-tracker.cpp:1018-1088, src/interpol.cpp:19-144) in their order and
 // without FMA contraction (this file is compiled with -fmad=false): the
-// interpolated values are computed in parallel, and its sums run over the
-// pattern points in point order, rounded after every point, as the
-// reference's loops round them; cos / sin come from ptk_crtrig.cuh.  Inside
-// Powell the frame region under the grain is staged in shared memory.
+// interpolated values are computed in parallel, and its sums are those of the
+// reference's loops over the pattern points in point order, rounded after
+// every point, computed by the whole block (ptk_seqsum.cuh); cos / sin come
+// from ptk_crtrig.cuh.  Inside Powell the frame region under the grain is
+// staged in shared memory.
 //
 // One CTA of kSubpixThreads refines one grain.  The Powell driver
 // (follow_pattern_subpixel_xyR, src/p-tracker.cpp:1090-1128; the minimiser
@@ -18,9 +19,11 @@
 // golden-ratio bracketing and Brent's parabolic line minimiser; its constants
 // and tests match the CPU oracle's restatement exactly.
 #include <climits>
+#include <type_traits>
 
 #include "ptk_crtrig.cuh"
 #include "ptk_internal.cuh"
+#include "ptk_seqsum.cuh"
 
 namespace ptk {
 
@@ -164,40 +167,194 @@ struct ObjGrain {
   double xref, yref;  // (double)refcoord + d, in the reference's order
   double drot;
   double mean0, c0c0;
-  int refx, refy;
 };
 
-// Current-frame region around a grain, staged once in shared memory for the
-// objective evaluations of its Powell run (uint16, row-major).  w == 0: none.
-struct Patch {
-  const uint16_t* pix;
-  int x0, y0, w, h;
-};
-
-__device__ __forceinline__ double patch_px(const Patch& pt, int x, int y) {
-  return (double)pt.pix[(y - pt.y0) * pt.w + (x - pt.x0)];
+// Exact integer -> double without the conversion pipe (a sixteenth of the
+// FP64 rate): the bits of 2^52 + v, minus 2^52.
+__device__ __forceinline__ double u16d(unsigned v) { return __hiloint2double(0x43300000, (int)v) - 0x1p52; }
+__device__ __forceinline__ double s32d(int v) {
+  return __hiloint2double(0x43300000, (int)((unsigned)v + 0x80000000u)) - (0x1p52 + 0x1p31);
+}
+// v / 2, exactly
+__device__ __forceinline__ double half_s32d(int v) {
+  return __hiloint2double(0x43200000, (int)((unsigned)v + 0x80000000u)) - (0x1p51 + 0x1p30);
 }
 
-// Per-grain state of the exact objective, in shared memory: the samples of
-// the last evaluation, the reference values under pattern0_rotated, and the
-// cosine and sine of the last rotation angle.
+// floor(x) and x - floor(x), both exact, for 0 <= x < 2^31: the nearest
+// integer in the low mantissa bits of x + 1.5 * 2^52, one less where it lies
+// above x.
+__device__ __forceinline__ double split(double x, int* ix) {
+  const double t = x + 0x1.8p52;
+  const double f = x - (t - 0x1.8p52);  // in [-0.5, 0.5]
+  const int below = __double2hiint(f) < 0 ? 1 : 0;  // (x an integer: f = +0)
+  *ix = __double2loint(t) - below;
+  return f + __hiloint2double(below ? 0x3ff00000 : 0, 0);
+}
+
+// cubic1 of four pixels at x (x2 = x * x): its coefficients are multiples of
+// 1/2 below 2^20, which cubic1's operations reach without rounding, so they
+// are formed as integers.
+__device__ __forceinline__ double cubic_px(int p0, int p1, int p2, int p3, double x, double x2) {
+  const double a = half_s32d(3 * (p1 - p2) + p3 - p0);
+  const double b = half_s32d(2 * p0 - 5 * p1 + 4 * p2 - p3);
+  const double c = half_s32d(p2 - p0);
+  return a * x2 * x + b * x2 + c * x + u16d((unsigned)p1);
+}
+
+// cubic1 with its multiplications by 2 and 1/2 folded: they are exact, so a
+// fused multiply-add by them rounds once, where the addition does.
+__device__ __forceinline__ double cubic1_fast(double p0, double p1, double p2, double p3, double x) {
+  const double t0 = p2 - p0, t1 = p3 - p1;  // 2 fp0, 2 fp1
+  const double c = 0.5 * t0;
+  const double b = __fma_rn(-0.5, t1, 3.0 * p2 - 3.0 * p1 - t0);
+  const double a = __fma_rn(0.5, t1, __fma_rn(2.0, p1 - p2, c));
+  const double x2 = x * x;
+  return a * x2 * x + b * x2 + c * x + p1;
+}
+
+// One block's grain and its exact objective, in shared memory: everything an
+// evaluation needs besides the point X.  The dynamic shared memory holds, per
+// pattern point, the sample of the current evaluation and, where they fit, the
+// centred reference value d0 = I0 - mean0 (doubles), and before them the
+// current-frame region around the grain (uint16, row-major, staged once; w = 0:
+// none).
 struct ExactObj {
-  const uint16_t* w0;    // P reference values (staged)
-  double* v;             // P interpolated values of the current evaluation (shared memory)
-  double* bcast;         // 8 doubles: [0] the evaluation's NCC, [3] cos, [4] sin, [5] C0C0
-  double inv_num_pix;    // 1 / P
-  double last_rot, c1, s1;
+  const short2* pat0;  // the grain's pattern points
+  const uint16_t* w0;  // and their reference values
+  FrameDev cur;
+  int interp, P;
+  SeqPlan one, two;    // how the sums' terms are split
+  double xref, yref, drot, mean0, c0c0, inv_num_pix;
+  double disp_max, stiffness;
+  int reach;           // every point lies within reach - 1 pixels of the pattern's origin
+  int x0, y0, w, h;    // the staged region
+  int v_at, d0_at;     // bytes from the start of the dynamic shared memory
+  int clamped;
+  double rot, c1, s1;  // the last rotation angle, its cosine and sine
+};
+__device__ __forceinline__ ExactObj& exact_obj() {
+  __shared__ ExactObj s;
+  return s;
+}
+extern __shared__ __align__(16) unsigned char s_subpix[];
+__device__ __forceinline__ double* obj_v(const ExactObj& ex) { return reinterpret_cast<double*>(s_subpix + ex.v_at); }
+__device__ __forceinline__ double* obj_d0(const ExactObj& ex) { return reinterpret_cast<double*>(s_subpix + ex.d0_at); }
+
+// Terms of the objective's sums, in point order (seq_sums).
+struct SumV {  // sum v
+  const double* v;
+  struct Of {
+    const double* v;
+    __device__ __forceinline__ double operator()(int i) const { return v[i]; }
+  };
+  __device__ __forceinline__ Of of(int) const { return Of{v}; }
+};
+// d0 of a point: staged, or from the reference value in global memory
+// (patterns whose values and d0 exceed the shared memory, and single
+// evaluations, which would read each staged value only three times).
+struct RefStaged {
+  const double* d0;
+  __device__ __forceinline__ explicit RefStaged(const ExactObj& ex) : d0(obj_d0(ex)) {}
+  __device__ __forceinline__ double operator()(int i) const { return d0[i]; }
+};
+struct RefGlobal {
+  const uint16_t* w0;
+  double mean0;
+  int last;
+  __device__ __forceinline__ explicit RefGlobal(const ExactObj& ex) : w0(ex.w0), mean0(ex.mean0), last(ex.P - 1) {}
+  __device__ __forceinline__ double operator()(int i) const { return u16d(w0[min(i, last)]) - mean0; }
+};
+template <class Ref>
+struct SumC {  // sum d0 d1 and sum d1^2
+  const double* d1;
+  Ref d0;
+  struct Of {
+    const double* d1;
+    Ref d0;
+    int n;
+    __device__ __forceinline__ double operator()(int i) const {
+      const double d = d1[i];
+      return (n == 0 ? d0(i) : d) * d;
+    }
+  };
+  __device__ __forceinline__ Of of(int n) const { return Of{d1, d0, n}; }
+};
+template <>
+struct SumC<RefStaged> {
+  const double* d1;
+  RefStaged d0;
+  struct Of {
+    const double *d1, *f;
+    __device__ __forceinline__ double operator()(int i) const { return f[i] * d1[i]; }
+  };
+  __device__ __forceinline__ Of of(int n) const { return Of{d1, n == 0 ? d0.d0 : d1}; }
+};
+template <class Ref>
+struct SumA {  // sum d0^2: C0C0 of do_precomputations (src/p-tracker.cpp:646-651)
+  Ref d0;
+  struct Of {
+    Ref d0;
+    __device__ __forceinline__ double operator()(int i) const {
+      const double d = d0(i);
+      return d * d;
+    }
+  };
+  __device__ __forceinline__ Of of(int) const { return Of{d0}; }
 };
 
-// Sum of d0_i^2 over the grain's points in point order, each step rounded:
-// C0C0 of do_precomputations (src/p-tracker.cpp:646-651).  One thread.
-__device__ double c0c0_in_order(const uint16_t* w0, int P, double mean0) {
-  double c = 0.0;
-  for (int i = 0; i < P; ++i) {
-    const double d0 = (double)w0[i] - mean0;
-    c += d0 * d0;
+// Samples of all points, by the block, where every 4x4 support lies in the
+// staged region.  Two points per thread at a time (their chains of dependent
+// operations, about 30 long, overlap), the next two's offsets loaded before.
+template <int NT, int KIND>
+__device__ __forceinline__ void sample_staged(const ExactObj& ex, double xpix1, double ypix1, double c1, double s1) {
+  constexpr int kAt = 2;
+  const uint16_t* patch = reinterpret_cast<const uint16_t*>(s_subpix);
+  double* v = obj_v(ex);
+  const short2* pat0 = ex.pat0;
+  const int P = ex.P, w = ex.w, at0 = -(ex.y0 + 1) * w - (ex.x0 + 1);
+  short2 q[kAt];
+#pragma unroll
+  for (int k = 0; k < kAt; ++k) q[k] = pat0[min((int)threadIdx.x + k * NT, P - 1)];
+  for (int i = threadIdx.x; i < P; i += kAt * NT) {
+    double x01[kAt], y01[kAt], val[kAt];
+    const uint16_t* px[kAt];
+#pragma unroll
+    for (int k = 0; k < kAt; ++k) {
+      const double x = s32d(q[k].x), y = s32d(q[k].y);
+      const double xs = xpix1 + c1 * x + s1 * y;
+      const double ys = ypix1 - s1 * x + c1 * y;
+      int ix, iy;
+      x01[k] = split(xs, &ix);
+      y01[k] = split(ys, &iy);
+      px[k] = patch + iy * w + ix + at0;  // the support's corner (ix - 1, iy - 1)
+      q[k] = pat0[min(i + (kAt + k) * NT, P - 1)];
+    }
+#pragma unroll
+    for (int k = 0; k < kAt; ++k) {
+      const uint16_t* p = px[k];
+      if constexpr (KIND == PTK_INTERP_LINEAR) {
+        const double a0 = u16d(p[w + 1]), a1 = u16d(p[2 * w + 1]), b0 = u16d(p[w + 2]), b1 = u16d(p[2 * w + 2]);
+        const double r0 = (a1 - a0) * y01[k] + a0;
+        const double r1 = (b1 - b0) * y01[k] + b0;
+        val[k] = (r1 - r0) * x01[k] + r0;
+      } else if constexpr (KIND == PTK_INTERP_CUBIC) {
+        const double y2 = y01[k] * y01[k];
+        double arr[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) arr[j] = cubic_px(p[j], p[w + j], p[2 * w + j], p[3 * w + j], y01[k], y2);
+        val[k] = cubic1_fast(arr[0], arr[1], arr[2], arr[3], x01[k]);
+      } else {
+        double arr[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          arr[j] = quintic1(u16d(p[j]), u16d(p[w + j]), u16d(p[2 * w + j]), u16d(p[3 * w + j]), y01[k]);
+        val[k] = quintic1(arr[0], arr[1], arr[2], arr[3], x01[k]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kAt; ++k)
+      if (i + k * NT < P) v[i + k * NT] = val[k];
   }
-  return c;
 }
 
 // NCC_to_minimize_xyR (src/p-tracker.cpp:1018-1088): the sample positions
@@ -205,83 +362,113 @@ __device__ double c0c0_in_order(const uint16_t* w0, int P, double mean0) {
 // reference's operations and order, every product and sum rounded separately
 // (this file is compiled without FMA contraction), cos / sin correctly
 // rounded (ptk_crtrig.cuh) where the host C library is within an ulp.  The
-// block's threads interpolate the points in parallel into shared memory; one
-// thread then runs the reference's two loops over them in point order,
+// block's threads interpolate the points in parallel into shared memory (82 FP64
+// operations a point, none of them a conversion, which runs at an eighth of
+// their rate: 206 operations' time before), then form the sums of the reference's two loops over them,
 //     mean1 = (sum v) * (1 / P),  C0C1 = sum d0 (v - mean1),  C1C1 = sum (v - mean1)^2
-// (d0 = I0 - mean0), each sum rounded after every point as the reference's
-// loops round it, so that the value is the reference's bit for bit and Powell
-// takes the reference's path even where the objective is flat.  Called by
-// every thread of the block with the same X; returns the same value on every
-// thread.
-template <int NT>
-__device__ double objective_exact(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp,
-                                  const ObjGrain& o, const Patch& pt, ExactObj& ex, const double X[3],
-                                  bool* clamped) {
+// (d0 = I0 - mean0), each rounded after every point in point order as those
+// loops round it (seq_sums), so that the value is the reference's bit for bit
+// and Powell takes the reference's path even where the objective is flat.
+// Called by every thread of the block with the same X; returns the same value
+// on every thread.  Not inlined: Powell calls it from a dozen places.
+template <int NT, class Ref>
+__device__ __noinline__ double objective_exact(double X0, double X1, double X2) {
+  ExactObj& ex = exact_obj();
   const int tid = threadIdx.x;
-  const double xpix1 = o.xref + X[0];
-  const double ypix1 = o.yref + X[1];
-  const double rot = o.drot + X[2];
-  if (!(rot == ex.last_rot)) {  // block-uniform: the line searches along x and y keep the angle
-    if (tid == 0) ex.bcast[3] = crtrig::cr_cos(rot);
-    if (tid == 32) ex.bcast[4] = crtrig::cr_sin(rot);
+  const double xpix1 = ex.xref + X0;
+  const double ypix1 = ex.yref + X1;
+  const double rot = ex.drot + X2;
+  if (!(rot == ex.rot)) {  // block-uniform: the line searches along x and y keep the angle
     __syncthreads();
-    ex.c1 = ex.bcast[3];
-    ex.s1 = ex.bcast[4];
-    ex.last_rot = rot;
+    if (tid == 0) {
+      ex.c1 = crtrig::cr_cos(rot);
+      ex.rot = rot;
+    }
+    if (tid == 32) ex.s1 = crtrig::cr_sin(rot);
+    __syncthreads();
   }
   const double c1 = ex.c1, s1 = ex.s1;
-  for (int i = tid; i < o.P; i += NT) {
-    const short2 q = g.pat0[o.b + i];
-    const double x = (double)q.x, y = (double)q.y;
-    const double xs = xpix1 + c1 * x + s1 * y;
-    const double ys = ypix1 - s1 * x + c1 * y;
-    double v;
-    const int ix = (int)floor(xs), iy = (int)floor(ys);
-    if (sp.interp == PTK_INTERP_CUBIC && pt.w > 0 && ix - 1 >= pt.x0 && iy - 1 >= pt.y0 && ix + 2 < pt.x0 + pt.w &&
-        iy + 2 < pt.y0 + pt.h) {
-      const double x01 = xs - (double)ix, y01 = ys - (double)iy;
-      double arr[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int xx = ix - 1 + k;
-        arr[k] = cubic1(patch_px(pt, xx, iy - 1), patch_px(pt, xx, iy), patch_px(pt, xx, iy + 1),
-                        patch_px(pt, xx, iy + 2), y01);
-      }
-      v = cubic1(arr[0], arr[1], arr[2], arr[3], x01);
-    } else {
-      v = interp(cur, sp.interp, xs, ys, clamped);
+  // block-uniform: every sample's 4x4 support lies in the staged region
+  const double reach = (double)ex.reach;
+  const bool inside = xpix1 - reach >= (double)(ex.x0 + 1) && ypix1 - reach >= (double)(ex.y0 + 1) &&
+                      xpix1 + reach <= (double)(ex.x0 + ex.w - 2) && ypix1 + reach <= (double)(ex.y0 + ex.h - 2);
+  if (inside) {
+    if (ex.interp == PTK_INTERP_CUBIC) sample_staged<NT, PTK_INTERP_CUBIC>(ex, xpix1, ypix1, c1, s1);
+    else if (ex.interp == PTK_INTERP_LINEAR) sample_staged<NT, PTK_INTERP_LINEAR>(ex, xpix1, ypix1, c1, s1);
+    else sample_staged<NT, PTK_INTERP_QUINTIC>(ex, xpix1, ypix1, c1, s1);
+  } else {
+    bool clamped = false;
+    double* v = obj_v(ex);
+    for (int i = tid; i < ex.P; i += NT) {
+      const short2 q = ex.pat0[i];
+      const double x = (double)q.x, y = (double)q.y;
+      const double xs = xpix1 + c1 * x + s1 * y;
+      const double ys = ypix1 - s1 * x + c1 * y;
+      v[i] = interp(ex.cur, ex.interp, xs, ys, &clamped);
     }
-    ex.v[i] = v;
+    if (clamped) ex.clamped = 1;
   }
   __syncthreads();
-  if (tid == 0) {
-    const double* v = ex.v;
-    double mean1 = 0.0;
-#pragma unroll 8
-    for (int i = 0; i < o.P; ++i) mean1 += v[i];
-    mean1 *= ex.inv_num_pix;
-    double c01 = 0.0, c11 = 0.0;
-#pragma unroll 8
-    for (int i = 0; i < o.P; ++i) {
-      const double d1 = v[i] - mean1;
-      const double d0 = (double)ex.w0[i] - o.mean0;
-      c01 += d0 * d1;
-      c11 += d1 * d1;
-    }
-    ex.bcast[0] = c01 / sqrt(o.c0c0 * c11);
+  const SeqSumScratch<NT>& sc = seq_scratch<NT>();
+  seq_sums<NT, 1>(ex.P, ex.one, SumV{obj_v(ex)});
+  __syncthreads();
+  const double mean1 = sc.out[0] * ex.inv_num_pix;
+  {  // d1 = v - mean1 in v's place
+    double* v = obj_v(ex);
+    for (int i = tid; i < ex.P; i += NT) v[i] -= mean1;
   }
   __syncthreads();
-  const double ncc = ex.bcast[0];
+  seq_sums<NT, 2>(ex.P, ex.two, SumC<Ref>{obj_v(ex), Ref(ex)});
+  __syncthreads();
+  const double ncc = sc.out[0] / sqrt(ex.c0c0 * sc.out[1]);
   double W = 1.0;
-  const double disp = sqrt(X[0] * X[0] + X[1] * X[1]);
-  if (disp > sp.disp_max) W = sp.stiffness * (disp - sp.disp_max) + 1.0;
+  const double d2 = X0 * X0 + X1 * X1;
+  if (!(ex.disp_max > 0.0 && d2 < 0.999999 * ex.disp_max * ex.disp_max)) {  // (well below it no root is needed)
+    const double disp = sqrt(d2);
+    if (disp > ex.disp_max) W = ex.stiffness * (disp - ex.disp_max) + 1.0;
+  }
   return (1.0 - ncc) * W;
 }
 
-// Once per grain: C0C0 as do_precomputations sums it (point order, each step
-// rounded; src/p-tracker.cpp:646-651) in bcast[5].  Every thread must call it.
-__device__ void grain_sums(const uint16_t* w0, int P, double mean0, double* bcast) {
-  if (threadIdx.x == 0) bcast[5] = c0c0_in_order(w0, P, mean0);
+// Sets the block's grain up and forms C0C0 in the reference's order.
+template <int NT, class Ref>
+__device__ __forceinline__ void exact_begin(const ObjGrain& o, const GrainsDev& g, const FrameDev& cur,
+                                            const SubpixParams& sp, int reach, int x0, int y0, int w, int h, int v_at,
+                                            int d0_at) {
+  ExactObj& ex = exact_obj();
+  if (std::is_same<Ref, RefStaged>::value) {
+    double* d0 = reinterpret_cast<double*>(s_subpix + d0_at);
+    for (int i = threadIdx.x; i < o.P; i += NT) d0[i] = u16d(g.w0[o.b + i]) - o.mean0;
+  }
+  if (threadIdx.x == 0) {
+    ex.pat0 = g.pat0 + o.b;
+    ex.w0 = g.w0 + o.b;
+    ex.mean0 = o.mean0;
+    ex.cur = cur;
+    ex.interp = sp.interp;
+    ex.P = o.P;
+    ex.one = seq_plan(o.P, NT);
+    ex.two = seq_plan(o.P, NT / 2);
+    ex.xref = o.xref;
+    ex.yref = o.yref;
+    ex.drot = o.drot;
+    ex.inv_num_pix = 1.0 / (double)o.P;
+    ex.disp_max = sp.disp_max;
+    ex.stiffness = sp.stiffness;
+    ex.reach = reach;
+    ex.x0 = x0;
+    ex.y0 = y0;
+    ex.w = w;
+    ex.h = h;
+    ex.v_at = v_at;
+    ex.d0_at = d0_at;
+    ex.clamped = 0;
+    ex.rot = __longlong_as_double(0x7ff8000000000000ll);
+  }
+  __syncthreads();
+  seq_sums<NT, 1>(o.P, ex.one, SumA<Ref>{Ref(ex)});
+  __syncthreads();
+  if (threadIdx.x == 0) ex.c0c0 = seq_scratch<NT>().out[0];
   __syncthreads();
 }
 
@@ -357,10 +544,8 @@ __device__ ObjGrain load_grain(const GrainsDev& g, int gi) {
   ObjGrain o;
   o.b = g.pstart[gi];
   o.P = g.pstart[gi + 1] - o.b;
-  o.refx = g.refx[gi];
-  o.refy = g.refy[gi];
-  o.xref = (double)o.refx + g.dx[gi];
-  o.yref = (double)o.refy + g.dy[gi];
+  o.xref = (double)g.refx[gi] + g.dx[gi];
+  o.yref = (double)g.refy[gi] + g.dy[gi];
   o.drot = g.drot[gi];
   o.mean0 = g.mean0[gi];
   o.c0c0 = g.c0c0[gi];
@@ -368,24 +553,17 @@ __device__ ObjGrain load_grain(const GrainsDev& g, int gi) {
 }
 
 // --- Powell on the device, block-uniform ----------------------------------
-template <int NT>
+template <int NT, class Ref>
 struct PowellEval {
-  const GrainsDev* g;
-  const FrameDev* cur;
-  const SubpixParams* sp;
-  const ObjGrain* o;
-  const Patch* pt;
-  ExactObj* ex;
-  bool* clamped;
-  int nfev;
-  __device__ double operator()(const double X[3]) {
-    ++nfev;
-    return objective_exact<NT>(*g, *cur, *sp, *o, *pt, *ex, X, clamped);
+  __device__ __forceinline__ double operator()(const double X[3]) const {
+    return objective_exact<NT, Ref>(X[0], X[1], X[2]);
   }
 };
 
+// f0: the objective at p, which is g(0): p + 0 dir is p bit for bit for finite
+// directions (p itself was reached as p + alpha dir, with the same roundings).
 template <class F>
-__device__ double line_minimize(F& f, const double p[3], const double dir[3], double* gmin) {
+__device__ double line_minimize(F& f, const double p[3], const double dir[3], double f0, double* gmin) {
   auto g = [&](double alpha) {
     double t[3];
 #pragma unroll
@@ -393,7 +571,7 @@ __device__ double line_minimize(F& f, const double p[3], const double dir[3], do
     return f(t);
   };
   double a = 0.0, b = 1.0;
-  double ga = g(a), gb = g(b);
+  double ga = isfinite(dir[0]) && isfinite(dir[1]) && isfinite(dir[2]) ? f0 : g(a), gb = g(b);
   if (gb > ga) {
     double t = a;
     a = b;
@@ -490,7 +668,7 @@ __device__ void powell_minimize(F& f, double p[3], const double step[3], double 
     for (int i = 0; i < 3; ++i) {
       const double fptt = fret;
       double gmin;
-      const double alpha = line_minimize(f, p, dirs[i], &gmin);
+      const double alpha = line_minimize(f, p, dirs[i], fret, &gmin);
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         dirs[i][j] *= alpha;
@@ -516,7 +694,7 @@ __device__ void powell_minimize(F& f, double p[3], const double step[3], double 
       const double t = 2.0 * (fp - 2.0 * fret + fe) * t1 * t1 - del * (fp - fe) * (fp - fe);
       if (t < 0.0) {
         double gmin;
-        const double alpha = line_minimize(f, p, xit, &gmin);
+        const double alpha = line_minimize(f, p, xit, fret, &gmin);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           xit[j] *= alpha;
@@ -537,9 +715,7 @@ __device__ void powell_minimize(F& f, double p[3], const double step[3], double 
 }  // namespace
 
 // Dynamic shared memory of the Powell kernel: the staged frame region (its
-// cap in uint16 elements first), then per pattern point its uint16 reference
-// value, then per pattern point the interpolated value of the current
-// evaluation (double).
+// cap in uint16 elements), then two doubles per pattern point.
 struct PowellSmem {
   int patch_cap;   // elements of the staged frame region
   int max_points;  // largest pattern of the grains
@@ -550,72 +726,62 @@ __host__ __device__ inline size_t powell_vals_offset(int patch_cap) {
   return ((size_t)patch_cap * sizeof(uint16_t) + 15) & ~(size_t)15;
 }
 
-// bytes of the staged reference values, padded so that the interpolated
-// values (doubles) after them stay 16-byte aligned
-__host__ __device__ inline size_t powell_w0_bytes(int max_points) {
-  return ((size_t)max_points * sizeof(uint16_t) + 15) & ~(size_t)15;
-}
+// after the last point's values: what the sums' walk may read past them
+constexpr size_t kTermPad = 4 * sizeof(double);
+
+// what a block may use besides the kernels' static shared memory
+constexpr size_t kPowellSmemMax = (227 - 12) * 1024;
+
+// Margin of the staged frame region around the pattern (pixels): the moves of
+// Powell's steps.  Samples further out read the frame.
+constexpr int kPatchMargin = 6;
 
 // follow_pattern_subpixel_xyR (src/p-tracker.cpp:1090-1128) for every grain,
 // one block per grain, grains taken in `order` (decreasing pattern size) when
-// given.
-__global__ void __launch_bounds__(kSubpixThreads, 3) k_subpix_powell(GrainsDev g, FrameDev cur, SubpixParams sp,
-                                                                       int patch_cap, int max_points,
-                                                                       const int* order, const int* list_count) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double bcast[8];
-  __shared__ int s_clamped, s_bb[4];
+// given.  A grain takes 160-400 evaluations one after another, so an
+// evaluation's latency counts: for 441 points 11.8k cycles (2.0k samples, 3.4k
+// the first sum, 4.7k the other two, 0.4k cosine and sine, 1.3k Powell's own
+// divisions and roots), against 33k with the sums and the cosine's series in one
+// thread.  Of whole pairs: 12 grains of up to 530 points 3.57 -> 1.95 ms, 400 of
+// 1,260-2,820 (8-bit frames of 2048x1536) 20.5 -> 7.7 ms, 2000 of up to 5,025
+// (5616x3744) 47.7 -> 27.2 ms of which the search takes 9.4.
+template <int NT, int BLOCKS, class Ref>
+__global__ void __launch_bounds__(NT, BLOCKS) k_subpix_powell(GrainsDev g, FrameDev cur, SubpixParams sp,
+                                                              int patch_cap, int max_points, const int* order,
+                                                              const int* list_count) {
+  __shared__ int s_m2;
   if (list_count && (int)blockIdx.x >= *list_count) return;
   const int gi = order ? order[blockIdx.x] : (int)blockIdx.x;
   if (g.masked[gi] || (g.flags[gi] & 3)) return;
-  ObjGrain o = load_grain(g, gi);
+  const ObjGrain o = load_grain(g, gi);
   if (o.P <= 0 || o.P > max_points) return;
   // stage the frame region under the pattern, with a margin for the Powell steps
-  if (threadIdx.x == 0) {
-    s_clamped = 0;
-    s_bb[0] = s_bb[2] = 1 << 30;
-    s_bb[1] = s_bb[3] = -(1 << 30);
-  }
+  if (threadIdx.x == 0) s_m2 = 0;
   __syncthreads();
-  uint16_t* s_patch = reinterpret_cast<uint16_t*>(smem);
-  uint16_t* s_w0 = reinterpret_cast<uint16_t*>(smem + powell_vals_offset(patch_cap));
-  double* s_v = reinterpret_cast<double*>(smem + powell_vals_offset(patch_cap) + powell_w0_bytes(max_points));
-  int xmn = 1 << 30, xmx = -(1 << 30), ymn = 1 << 30, ymx = -(1 << 30);
-  for (int i = threadIdx.x; i < o.P; i += kSubpixThreads) {
+  const int v_at = (int)powell_vals_offset(patch_cap), d0_at = v_at + max_points * (int)sizeof(double);
+  uint16_t* s_patch = reinterpret_cast<uint16_t*>(s_subpix);
+  int m2 = 0;
+  for (int i = threadIdx.x; i < o.P; i += NT) {
     const short2 q = g.pat0[o.b + i];
-    xmn = min(xmn, (int)q.x);
-    xmx = max(xmx, (int)q.x);
-    ymn = min(ymn, (int)q.y);
-    ymx = max(ymx, (int)q.y);
-    s_w0[i] = g.w0[o.b + i];
+    m2 = max(m2, (int)q.x * q.x + (int)q.y * q.y);
   }
-  atomicMin(&s_bb[0], xmn);
-  atomicMax(&s_bb[1], xmx);
-  atomicMin(&s_bb[2], ymn);
-  atomicMax(&s_bb[3], ymx);
+  atomicMax(&s_m2, m2);
   __syncthreads();
-  constexpr int kMargin = 6;
+  const int reach = (int)ceil(sqrt((double)s_m2)) + 1;
   const int cx = (int)floor(o.xref), cy = (int)floor(o.yref);
-  int px0 = max(cx + s_bb[0] - kMargin, 0), py0 = max(cy + s_bb[2] - kMargin, 0);
-  int px1 = min(cx + s_bb[1] + kMargin + 2, cur.dimx), py1 = min(cy + s_bb[3] + kMargin + 2, cur.dimy);
+  const int px0 = max(cx - reach - kPatchMargin, 0), py0 = max(cy - reach - kPatchMargin, 0);
+  const int px1 = min(cx + reach + kPatchMargin + 3, cur.dimx), py1 = min(cy + reach + kPatchMargin + 3, cur.dimy);
   int pw = max(px1 - px0, 0), ph = max(py1 - py0, 0);
   if (pw * ph > patch_cap) ph = pw > 0 ? min(ph, patch_cap / pw) : 0;  // samples outside read the frame
-  for (int e = threadIdx.x; e < pw * ph; e += kSubpixThreads) {
+  for (int e = threadIdx.x; e < pw * ph; e += NT) {
     const int yy = e / pw, xx = e - yy * pw;
     s_patch[e] = cur.pix[(size_t)(py0 + yy) * cur.pitch + (px0 + xx)];
   }
-  __syncthreads();
-  grain_sums(s_w0, o.P, o.mean0, bcast);
-  o.c0c0 = bcast[5];
-  const Patch pt{s_patch, px0, py0, pw, ph};
-  ExactObj ex{s_w0, s_v, bcast, 1.0 / (double)o.P, __longlong_as_double(0x7ff8000000000000ll), 0.0, 0.0};
-  bool clamped = false;
-  PowellEval<kSubpixThreads> f{&g, &cur, &sp, &o, &pt, &ex, &clamped, 0};
+  exact_begin<NT, Ref>(o, g, cur, sp, reach, px0, py0, pw, ph, v_at, d0_at);
+  const PowellEval<NT, Ref> f{};
   double X[3] = {0.0, 0.0, 0.0};
   double fret;
   powell_minimize(f, X, sp.init_dir, sp.tol, &fret);
-  if (clamped) atomicOr(&s_clamped, 1);
-  __syncthreads();
   if (threadIdx.x == 0) {
     g.ncc_subpix[gi] = 1.0 - fret;
     g.upix[gi] += X[0];
@@ -624,91 +790,113 @@ __global__ void __launch_bounds__(kSubpixThreads, 3) k_subpix_powell(GrainsDev g
     g.dx[gi] += X[0];
     g.dy[gi] += X[1];
     g.drot[gi] += X[2];
-    if (s_clamped) g.status[gi] |= PTK_ST_SUBPIX_CLAMPED;
+    if (exact_obj().clamped) g.status[gi] |= PTK_ST_SUBPIX_CLAMPED;
   }
 }
 
-// Objective (the exact one, as Powell evaluates it) or its FP64 gradient at
-// caller-given X for every grain.
+// Objective at caller-given X for every grain, as Powell evaluates it.
 __global__ void __launch_bounds__(kSubpixThreads) k_objective(GrainsDev g, FrameDev cur, SubpixParams sp,
-                                                                const double* Xall, double* f, double* grad,
-                                                                int max_points) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[kSubpixThreads / 32];
-  __shared__ double bcast[8];
+                                                                const double* Xall, double* f, int max_points) {
   const int gi = blockIdx.x;
-  ObjGrain o = load_grain(g, gi);
+  const ObjGrain o = load_grain(g, gi);
   if (o.P <= 0 || o.P > max_points) {
-    if (threadIdx.x == 0) {
-      f[gi] = __longlong_as_double(0x7ff8000000000000ll);
-      if (grad) grad[3 * gi] = grad[3 * gi + 1] = grad[3 * gi + 2] = f[gi];
-    }
+    if (threadIdx.x == 0) f[gi] = __longlong_as_double(0x7ff8000000000000ll);
     return;
   }
-  double* vals = reinterpret_cast<double*>(smem);
-  const double X[3] = {Xall[3 * gi], Xall[3 * gi + 1], Xall[3 * gi + 2]};
-  bool clamped = false;
-  double val;
-  if (grad) {
-    double G[3];
-    val = objective_grad<kSubpixThreads>(g, cur, sp, o, X, vals, red, G, &clamped);
-    if (threadIdx.x == 0) {
-      grad[3 * gi] = G[0];
-      grad[3 * gi + 1] = G[1];
-      grad[3 * gi + 2] = G[2];
-    }
-  } else {
-    uint16_t* s_w0 = reinterpret_cast<uint16_t*>(smem);
-    double* s_v = reinterpret_cast<double*>(smem + powell_w0_bytes(max_points));
-    for (int i = threadIdx.x; i < o.P; i += kSubpixThreads) s_w0[i] = g.w0[o.b + i];
-    __syncthreads();
-    grain_sums(s_w0, o.P, o.mean0, bcast);
-    o.c0c0 = bcast[5];
-    const Patch none{nullptr, 0, 0, 0, 0};
-    ExactObj ex{s_w0, s_v, bcast, 1.0 / (double)o.P, __longlong_as_double(0x7ff8000000000000ll), 0.0, 0.0};
-    val = objective_exact<kSubpixThreads>(g, cur, sp, o, none, ex, X, &clamped);
-  }
+  // one evaluation: no frame region is staged
+  exact_begin<kSubpixThreads, RefGlobal>(o, g, cur, sp, 0, 0, 0, 0, 0, 0, 0);
+  const double val = objective_exact<kSubpixThreads, RefGlobal>(Xall[3 * gi], Xall[3 * gi + 1], Xall[3 * gi + 2]);
   if (threadIdx.x == 0) f[gi] = val;
 }
 
-static PowellSmem powell_smem(int max_points, int max_r) {
+// The objective's FP64 gradient (and value, in block order) at caller-given X
+// for every grain.
+__global__ void __launch_bounds__(kSubpixThreads) k_objective_grad(GrainsDev g, FrameDev cur, SubpixParams sp,
+                                                                     const double* Xall, double* f, double* grad,
+                                                                     int max_points) {
+  __shared__ double red[kSubpixThreads / 32];
+  const int gi = blockIdx.x;
+  const ObjGrain o = load_grain(g, gi);
+  if (o.P <= 0 || o.P > max_points) {
+    if (threadIdx.x == 0)
+      f[gi] = grad[3 * gi] = grad[3 * gi + 1] = grad[3 * gi + 2] = __longlong_as_double(0x7ff8000000000000ll);
+    return;
+  }
+  const double X[3] = {Xall[3 * gi], Xall[3 * gi + 1], Xall[3 * gi + 2]};
+  bool clamped = false;
+  double G[3];
+  const double val = objective_grad<kSubpixThreads>(g, cur, sp, o, X, reinterpret_cast<double*>(s_subpix), red, G,
+                                                     &clamped);
+  if (threadIdx.x == 0) {
+    f[gi] = val;
+    grad[3 * gi] = G[0];
+    grad[3 * gi + 1] = G[1];
+    grad[3 * gi + 2] = G[2];
+  }
+}
+
+// `staged`: the centred reference values too (powell_staged).
+static PowellSmem powell_smem(int max_points, int max_r, bool staged) {
   PowellSmem m;
-  const size_t side = (size_t)(2 * max_r + 1 + 2 * 6 + 2);
+  // the reach of a rotated and rounded pattern is at most max_r + 1
+  const size_t side = (size_t)(2 * (max_r + 1) + 2 * kPatchMargin + 3);
   size_t patch = side * side;
-  const size_t rest = powell_w0_bytes(max_points) + (size_t)max_points * sizeof(double);
-  constexpr size_t kCap = 227 * 1024 - 1024;  // the kernel's static shared memory included
-  if (powell_vals_offset((int)patch) + rest > kCap)
-    patch = rest < kCap ? (kCap - rest) / sizeof(uint16_t) - 8 : 0;  // samples outside the region read the frame
+  const size_t rest = (size_t)max_points * sizeof(double) * (staged ? 2 : 1);
+  if (powell_vals_offset((int)patch) + rest > kPowellSmemMax)  // samples outside the region read the frame
+    patch = rest < kPowellSmemMax ? (kPowellSmemMax - rest) / sizeof(uint16_t) - 8 : 0;
   m.patch_cap = (int)patch;
   m.max_points = max_points;
-  m.bytes = powell_vals_offset(m.patch_cap) + rest;
+  m.bytes = powell_vals_offset(m.patch_cap) + rest + kTermPad;
   return m;
 }
 
-void prepare_subpix(int max_points, int max_r) {
-  const PowellSmem m = powell_smem(max_points, max_r);
-  ensure_smem((const void*)k_subpix_powell, m.bytes);
-  // the objective alone: reference and interpolated values; with the gradient: three doubles per point
-  const size_t bf = powell_w0_bytes(max_points) + (size_t)max_points * sizeof(double);
-  const size_t bg = (size_t)max_points * sizeof(double) * 3;
-  ensure_smem((const void*)k_objective, bg <= 227 * 1024 && bg > bf ? bg : bf);
+static bool powell_staged(int max_points) { return (size_t)max_points * 2 * sizeof(double) <= kPowellSmemMax - 32 * 1024; }
+
+// The kernel of a launch.  128 threads a block, except where there are no more
+// grains than SMs (each block has an SM to itself, and its evaluations'
+// latency is the whole time) and patterns large enough to keep 256 busy: 80
+// grains of up to 5,000 points 18.9 -> 17.4 ms, 40 of up to 2,100 equal, 12 of
+// up to 530 1.88 -> 2.11 ms, 2000 grains of up to 5,000 27.4 -> 28.9 ms.
+constexpr int kPowellWidePoints = 1500;
+typedef void (*PowellKernel)(GrainsDev, FrameDev, SubpixParams, int, int, const int*, const int*);
+static PowellKernel powell_kernel(int n, int max_points, int num_sms, int* threads) {
+  if (!powell_staged(max_points)) {
+    *threads = 256;
+    return k_subpix_powell<256, 1, RefGlobal>;
+  }
+  const bool wide = n <= num_sms && max_points > kPowellWidePoints;
+  *threads = wide ? 256 : 128;
+  return wide ? k_subpix_powell<256, 2, RefStaged> : k_subpix_powell<128, 3, RefStaged>;
 }
 
-void launch_subpix_powell(const GrainsDev& g, const FrameDev& cur, const FrameDev& /*ref*/, const SubpixParams& sp,
-                          int max_points, int max_r, const int* order, cudaStream_t s, const int* list_count) {
+void prepare_subpix(int n, int max_points, int max_r, int num_sms) {
+  int threads;
+  const PowellKernel k = powell_kernel(n, max_points, num_sms, &threads);
+  ensure_smem((const void*)k, powell_smem(max_points, max_r, powell_staged(max_points)).bytes);
+}
+
+void launch_subpix_powell(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, int max_points, int max_r,
+                          int num_sms, const int* order, cudaStream_t s, const int* list_count) {
   if (g.n <= 0) return;
-  prepare_subpix(max_points, max_r);
-  const PowellSmem m = powell_smem(max_points, max_r);
-  k_subpix_powell<<<g.n, kSubpixThreads, m.bytes, s>>>(g, cur, sp, m.patch_cap, max_points, order, list_count);
+  prepare_subpix(g.n, max_points, max_r, num_sms);
+  int threads;
+  const PowellKernel k = powell_kernel(g.n, max_points, num_sms, &threads);
+  const PowellSmem m = powell_smem(max_points, max_r, powell_staged(max_points));
+  k<<<g.n, threads, m.bytes, s>>>(g, cur, sp, m.patch_cap, max_points, order, list_count);
 }
 
 void launch_objective(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const double* X, double* f,
                       double* grad, int max_points, cudaStream_t s) {
   if (g.n <= 0) return;
-  prepare_subpix(max_points, 0);
-  const size_t smem = grad ? (size_t)max_points * sizeof(double) * 3
-                           : powell_w0_bytes(max_points) + (size_t)max_points * sizeof(double);
-  k_objective<<<g.n, kSubpixThreads, smem, s>>>(g, cur, sp, X, f, grad, max_points);
+  // with the gradient: its samples too
+  const size_t bytes = (size_t)max_points * sizeof(double) * (grad ? 3 : 1) + (grad ? 0 : kTermPad);
+  if (grad) {
+    if (bytes <= 227 * 1024) ensure_smem((const void*)k_objective_grad, bytes);
+    k_objective_grad<<<g.n, kSubpixThreads, bytes, s>>>(g, cur, sp, X, f, grad, max_points);
+  } else {
+    ensure_smem((const void*)k_objective, bytes);
+    k_objective<<<g.n, kSubpixThreads, bytes, s>>>(g, cur, sp, X, f, max_points);
+  }
 }
 
 }  // namespace ptk

@@ -1,0 +1,86 @@
+"""The plain objective's sums, formed by a whole block, against the oracle's
+serial loops: equal bit for bit.  Rotation 0 (cosine 1 and sine 0 on both sides)
+and displacements in quarters of a pixel, so that samples have few bits and
+ties abound; pattern sizes around the kernel's splits (chunks of 1 + 4 l points,
+64 or 128 threads a sum) and the largest allowed; frames whose sums change
+binade and sign in every way."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIZES = (1, 2, 5, 63, 64, 65, 127, 128, 129, 319, 320, 321, 639, 641, 1153, 2000, 5025, 16384)
+
+
+def _frames(kind: str, rng):
+    ref = rng.integers(0, 65536, (320, 320)).astype(np.uint16)
+    if kind == "random":       # sums of the cross term that wander about zero
+        cur = rng.integers(0, 65536, ref.shape).astype(np.uint16)
+    elif kind == "match":
+        cur = ref.copy()
+    elif kind == "negative":   # an anticorrelated window: falling sums
+        cur = (65535 - ref).astype(np.uint16)
+    elif kind == "steps":      # zeros first, then ever larger values: many binades
+        ramp = np.minimum(2 ** (np.arange(320) // 20), 65535).astype(np.uint16)
+        cur = np.where(rng.random(ref.shape) < 0.5, 0, ramp[:, None]).astype(np.uint16)
+        ref = np.where(rng.random(ref.shape) < 0.3, ref, 7).astype(np.uint16)
+    else:                      # "flat": no variance, the value is not a number
+        cur = np.full(ref.shape, 1000, dtype=np.uint16)
+    return ref, cur
+
+
+@pytest.mark.parametrize("kind", ["random", "match", "negative", "steps", "flat"])
+def test_objective_is_the_serial_loop(ptk, oracle, cuda_device, kind):
+    rng = np.random.default_rng(len(kind))
+    ref, cur = _frames(kind, rng)
+    grid = np.stack(np.meshgrid(np.arange(-64, 64), np.arange(-64, 64)), -1).reshape(-1, 2)
+    pats = [grid[rng.permutation(len(grid))[:P]] if P < 16384 else grid for P in SIZES]
+    n = len(SIZES)
+    rec = np.zeros((n, 13))
+    rec[:, 0], rec[:, 1], rec[:, 3] = 160, 160, 64
+    t = ptk.Tracker(320, 320)
+    t.set_grains(rec)
+    t.set_patterns(pats)
+    t.load_frame(0, ref)
+    t.load_frame(1, cur)
+    t.precompute()
+    c = oracle.Port(320, 320, 1)
+    c.load_first(ref)
+    c.load_current(cur)
+    c.set_grains(rec)
+    for g, p in enumerate(pats):
+        c.set_pattern(g, p)
+    c.precompute()
+    for X in ((0.0, 0.0, 0.0), (0.5, -0.25, 0.0), (-0.75, 0.5, 0.0), (1.3, 2.1, 0.0)):
+        got = t.objective(np.tile(X, (n, 1)))
+        want = np.array([c.objective(g, X) for g in range(n)])
+        np.testing.assert_array_equal(got, want)
+    t.close()
+
+
+@pytest.mark.parametrize("n,interp", [(40, "cubic"), (200, "cubic"), (40, "linear"), (40, "quintic")])
+def test_refinement_takes_the_reference_path(ptk, wl, oracle, cuda_device, n, interp):
+    """Powell's result bit for bit (both kernel widths: fewer grains than SMs
+    and more), on the grains whose angles the C library rounds correctly: about
+    one sine in 420 is not, and a grain visits some 100 angles, so that about
+    0.79 of the grains are expected to be equal; the others stay within 1e-5 px."""
+    p = dict(wl.PRESETS["small16"], dimx=1536, dimy=1024, n=n, mix=[(0.5, 8.0, 18.0), (0.5, 22.0, 30.0)])
+    pair = wl.make_pair(p, seed=5)
+    o = wl.tracker_options(p)
+    t = ptk.Tracker(p["dimx"], p["dimy"], image_interpolator=interp, iraz=100, **o)
+    t.set_grains(pair["rec"])
+    t.make_patterns("grain_diameter", 1.0, 1.0)
+    t.load_frame(0, pair["ref"])
+    t.load_frame(1, pair["cur"])
+    t.track_frame(1)
+    got = t.get_grains()
+    c = oracle.setup(oracle.Port, pair, threads=8, zones=o["zones"],
+                     params={"rescue_level": 0, "NCC_min": 0.7, "iraz": 100, "image_interpolator": ptk.INTERP[interp]})
+    c.track_frame(1)
+    want = c.get_grains()
+    same = (got[:, 4:7] == want[:, 4:7]).all(axis=1)
+    assert same.mean() >= 0.5, same.mean()
+    assert np.abs(got[:, 4:6] - want[:, 4:6]).max() <= 1e-5
+    t.close()
