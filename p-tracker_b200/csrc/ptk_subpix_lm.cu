@@ -17,6 +17,12 @@
 // damped normal equations are solved in FP64 and X and the cumulative grain
 // state accumulate in FP64.
 //
+// What bounds it: an evaluation's latency, which besides the points is the
+// reduction (18 FP64 sums) and the divisions of the normal equations (some 400
+// cycles each), so the sums are spread over the lanes while they are reduced and
+// the divisions are taken one per lane: 2000 grains of up to 5,025 points 185 ->
+// 160 us, 40 of up to 2,100 44.7 -> 40.7 us, same bits.
+//
 // One 128-thread block per grain, grains in decreasing pattern size (the
 // level-0 order) so that the large ones start first; the iteration stops when
 // the step is below the tolerance, or after two rejected steps in a row once
@@ -162,40 +168,67 @@ __device__ LmEval lm_eval(const GrainsDev& g, const FrameDev& cur, const LmPatch
     S[16] += a * gy;
     S[17] += a * gr;
   }
-  // warp sums in FP64, then the warps' partial sums in index order
+  // Warp sums in FP64 by a butterfly over the lanes, in which each lane keeps
+  // and adds only the half of the values that it is responsible for (20
+  // exchanges instead of the 90 of 18 full butterflies; every value's additions
+  // are the same): lane l ends with value `k`, if any.
+  double t[kNSums];
 #pragma unroll
-  for (int k = 0; k < kNSums; ++k) {
-    double t = k == 0 ? S0 : (k == 1 ? S1 : (k == 2 ? S2 : (double)S[k]));
-    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
-    if (lane == 0) part[warp][k] = t;
+  for (int k = 0; k < kNSums; ++k) t[k] = k == 0 ? S0 : (k == 1 ? S1 : (k == 2 ? S2 : (double)S[k]));
+  {
+    int n = kNSums;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const int m = (n + 1) / 2;
+      const bool up = (lane & off) != 0;
+#pragma unroll
+      for (int k = 0; k < (kNSums + 1) / 2; ++k)
+        if (k < m) {
+          const double lo = t[k], hi = k + m < n ? t[k + m] : 0.0;
+          t[k] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, off);
+        }
+      n = m;
+    }
+    const int p4 = (lane & 1) + (lane & 2), p3 = p4 + ((lane & 4) ? 3 : 0), p2 = p3 + ((lane & 8) ? 5 : 0);
+    const int k = p2 + ((lane & 16) ? 9 : 0);
+    if (p4 < 3 && p3 < 5 && p2 < 9) part[warp][k] = t[0];
   }
   const int any_clamped = __syncthreads_or(clamped ? 1 : 0);
-  double T[kNSums];
-#pragma unroll
-  for (int k = 0; k < kNSums; ++k) {
-    double t = part[0][k];
-    for (int w = 1; w < NT / 32; ++w) t += part[w][k];
-    T[k] = t;
+  if (tid < kNSums) {  // the warps' partial sums in index order, in the last row
+    double sum = part[0][tid];
+    for (int w = 1; w < NT / 32; ++w) sum += part[w][tid];
+    part[NT / 32][tid] = sum;
   }
-  __syncthreads();  // part[] is rewritten by the next evaluation
+  __syncthreads();
+  const double* T = part[NT / 32];  // (written again after the next evaluation's first barrier)
   LmEval e;
   e.clamped = any_clamped != 0;
+  // The divisions one per lane: each takes some 400 cycles, and there are 19.
   const double P = (double)o.P;
   const double mv = T[0] / P;
   const double n2 = T[1] - P * mv * mv;  // sum b^2
   const double n = sqrt(n2);
-  // sum a = 0 up to rounding, so sum a b = sum a vc
-  e.ncc = T[2] / (o.norm_a * n);
+  // lane: 0-2 gbar = sum g / P, 3-5 c = (sum b g) / n, 6-8 (sum a g) / |a|, 9 the NCC
+  // (sum a = 0 up to rounding, so sum a b = sum a vc)
+  const int j = lane < 9 ? lane % 3 : 0;
+  const double c_num = T[12 + j] - mv * T[3 + j];
+  const double q_num = lane < 3 ? T[3 + j] : (lane < 6 ? c_num : (lane < 9 ? T[15 + j] : T[2]));
+  const double q_den = lane < 3 ? P : (lane < 6 ? n : (lane < 9 ? o.norm_a : o.norm_a * n));
+  const double q = q_num / q_den;
+  e.ncc = __shfl_sync(0xffffffffu, q, 9);
   e.F = 2.0 * (1.0 - e.ncc);
-  const double gb[3] = {T[3] / P, T[4] / P, T[5] / P};
-  const double cc[3] = {(T[12] - mv * T[3]) / n, (T[13] - mv * T[4]) / n, (T[14] - mv * T[5]) / n};
-  const double gg[6] = {T[6], T[7], T[8], T[9], T[10], T[11]};
-  const int ia[6] = {0, 0, 0, 1, 1, 2}, ib[6] = {0, 1, 2, 1, 2, 2};
+  // lane: 0-5 H (xx, xy, xr, yy, yr, rr), 6-8 the gradient
+  const int ia = lane < 3 ? 0 : (lane < 5 ? 1 : 2), ib = lane < 3 ? lane : (lane < 5 ? lane - 2 : 2);
+  const double ga = __shfl_sync(0xffffffffu, q, ia), gb = __shfl_sync(0xffffffffu, q, ib);
+  const double ca = __shfl_sync(0xffffffffu, q, 3 + ia), cb = __shfl_sync(0xffffffffu, q, 3 + ib);
+  const double cj = __shfl_sync(0xffffffffu, q, 3 + j);
+  const double h_num = T[6 + (lane < 6 ? lane : 0)] - P * ga * gb - ca * cb;
+  const double g_num = q - cj * e.ncc;  // (lanes 6-8: q is (sum a g) / |a|)
+  const double r = (lane < 6 ? h_num : g_num) / (lane < 6 ? n2 : n);
 #pragma unroll
-  for (int k = 0; k < 6; ++k) e.H[k] = (gg[k] - P * gb[ia[k]] * gb[ib[k]] - cc[ia[k]] * cc[ib[k]]) / n2;
-  const double ga[3] = {T[15] / o.norm_a, T[16] / o.norm_a, T[17] / o.norm_a};
+  for (int k = 0; k < 6; ++k) e.H[k] = __shfl_sync(0xffffffffu, r, k);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) e.gv[k] = -(ga[k] - cc[k] * e.ncc) / n;
+  for (int k = 0; k < 3; ++k) e.gv[k] = -__shfl_sync(0xffffffffu, r, 6 + k);
   return e;
 }
 
@@ -254,7 +287,7 @@ __device__ LmPatch lm_stage(const GrainsDev& g, const FrameDev& cur, const LmGra
 
 __global__ void __launch_bounds__(kLmThreads) k_subpix_lm(GrainsDev g, FrameDev cur, LmParams lp, int patch_cap) {
   extern __shared__ __align__(16) float s_lm_patch[];
-  __shared__ double part[kLmThreads / 32][kNSums];
+  __shared__ double part[kLmThreads / 32 + 1][kNSums];
   __shared__ int s_bb[4];
   const int gi = lp.order ? lp.order[blockIdx.x] : (int)blockIdx.x;
   if (g.masked[gi] || (g.flags[gi] & 3)) return;
@@ -331,7 +364,7 @@ __global__ void __launch_bounds__(kLmThreads) k_subpix_lm(GrainsDev g, FrameDev 
 // F = 1 - NCC and its gradient from the FP32 adjoint sums (for checks).
 __global__ void __launch_bounds__(kLmThreads) k_grad_f32(GrainsDev g, FrameDev cur, const double* Xall, double* f,
                                                         double* grad) {
-  __shared__ double part[kLmThreads / 32][kNSums];
+  __shared__ double part[kLmThreads / 32 + 1][kNSums];
   const int gi = blockIdx.x;
   LmGrain o;
   o.b = g.pstart[gi];
