@@ -613,6 +613,8 @@ int enqueue_search(ptk_ctx* c, int level, cudaStream_t s, cudaEvent_t* ev = null
     b.down = z.down;
     b.tiles_u = sg.tiles_u;
     b.tiles_v = sg.tiles_v;
+    b.nx = std::min(4, (sg.nu + 7) / 8);
+    b.ny = std::min(kTileV, (sg.nv + 1) & ~1);
     b.keep = std::min(std::max(c->cfg.topk, 1), kBf16KeepMax);
     b.max_items = (int)sg.items;
     b.half = c->d_bf_half;

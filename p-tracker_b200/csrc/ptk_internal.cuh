@@ -110,6 +110,7 @@ struct Bf16Launch {
   int nrot;
   int left, right, up, down;
   int tiles_u, tiles_v;
+  int nx, ny;               // a tile's 8-column x shifts (1..4) and y offsets (even, 2..32) that any of the zone's tiles needs
   int keep;                 // candidates per tile rescored exactly (1..kBf16KeepMax)
   int max_items;            // list capacity x tiles: grid of the per-tile kernels
   const int* half;          // per grain: footprint half-extent ceil(max |offset|) + 1

@@ -40,8 +40,12 @@
 //     no multicast), one per footprint row and operand: the rotation slots
 //     beyond the level's steps come along and feed accumulator lanes that
 //     are never read.
-//   * B operands (N = 256 = 32 y offsets by 8 x offsets, K = 16 image
-//     columns): the current frame minus m, and its square, in a Hankel
+//   * B operands (N = 8 ny = ny y offsets by 8 x offsets, K = 16 image columns;
+//     ny = 32, or the zone's height, made even, where that is less: an MMA's
+//     time is proportional to N, and the shifts beyond the zone's width save
+//     their last chunk.  Zone +-6, 40
+//     grains of up to 2,100 points: 70.6 -> 58.3 us; +-8, 400 grains: 204 -> 174
+//     us; with the issue loop below 45.1 and 139): the current frame minus m, and its square, in a Hankel
 //     layout - per image row and 8-column block, 8 entries of 16 bytes, entry
 //     s holding the 8 pixels that start s columns into the block - so the 8 x
 //     offsets of a core matrix are 16 bytes apart, K halves 128 bytes apart
@@ -105,6 +109,7 @@ constexpr int kStageBoxRows = 8;  // image rows per TMA box of the strip staging
 // (they complete unless the device is broken) get a longer bound
 constexpr long kDrainLimit = 1L << 26;
 // operand rows in flight: W_r and M_r of one footprint row per ring buffer
+constexpr int kRowThread = 32;  // issues the operand rows' copies during the MMA phases
 constexpr int kRing = 8;       // barrier slots
 constexpr int kRingUsed = 4;   // buffers
 // weights kernel: 512 threads, 108 KB of 32-bit maps (two blocks per SM, as
@@ -112,15 +117,16 @@ constexpr int kRingUsed = 4;   // buffers
 constexpr int kWThreads = 512;
 constexpr int kWSmem = 108 * 1024;
 
-// A and B operand formats: BF16 x BF16 -> FP32, both K-major, M = 128, N = 256.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) |
-                            ((uint32_t)(128 >> 4) << 24);
+// A and B operand formats: BF16 x BF16 -> FP32, both K-major, M = 128, N = 8 ny.
+__host__ __device__ constexpr uint32_t idesc_of(int ny) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)ny << 17) | ((uint32_t)(128 >> 4) << 24);
+}
 
 struct Geom {
   int half;  // footprint covers offsets [-half, half] in x and y
   int fw;    // footprint side
   int nbf;   // 8-column blocks of the footprint
-  int nch;   // 16-column MMA chunks (footprint + 24 columns of shift)
+  int nch;   // 16-column MMA chunks (footprint + 8 (nx - 1) columns of shift)
   int wb;    // weight blocks per row in shared memory (3 leading zero blocks)
   int hb;    // Hankel blocks per image row
   int rp;    // bytes per staged image row (8 hb + 16 pixels from a 16-byte boundary: one TMA box row)
@@ -128,19 +134,21 @@ struct Geom {
   int nb;    // operand-row ring buffers
 };
 
-__host__ __device__ inline Geom geom_of(int half, int nb = kRingUsed) {
+// nx, ny: x shifts and y offsets of a tile (Bf16Launch)
+__host__ __device__ inline Geom geom_of(int half, int nb = kRingUsed, int nx = 4, int ny = kTileV) {
   Geom g;
   g.half = half;
   g.fw = 2 * half + 1;
   g.nbf = (g.fw + 7) / 8;
-  g.nch = (g.nbf + 3 + 1) / 2;
+  g.nch = (g.nbf + nx) / 2;
+  if (g.nch < 2) g.nch = 2;
   g.wb = 2 * g.nch + 3;
   g.hb = 2 * g.nch;
   g.rp = 16 * g.hb + 32;
   // the operand-row ring, then two Hankel buffers and the staged image rows
-  // with 31 rows of halo (staged in boxes of 8 rows: up to 7 more)
+  // with ny - 1 rows of halo (staged in boxes of 8 rows: up to 7 more)
   const int halo_row = 2 * g.hb * 128 + g.rp;
-  int rs = (kSmemBudget - nb * 2 * g.wb * 512 - (kStageBoxRows - 1) * g.rp) / halo_row - 31;
+  int rs = (kSmemBudget - nb * 2 * g.wb * 512 - (kStageBoxRows - 1) * g.rp) / halo_row - (ny - 1);
   if (rs > g.fw) rs = g.fw;
   g.rs = rs < 1 ? 1 : rs;
   g.nb = nb;
@@ -158,11 +166,12 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(dtmem),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
@@ -430,8 +439,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
   __shared__ __align__(8) unsigned long long s_probe;  // failure-path test: nothing ever arrives on it
   __shared__ __align__(8) unsigned long long s_stage;  // a strip's image rows staged (TMA)
   __shared__ int s_stage_out;                          // stagings issued and not yet waited for (0 or 1)
-  // operand rows through the ring (thread 0): uses of each buffer copied and
-  // consumed so far (a buffer's barriers complete one phase per use)
+  // operand rows through the ring: uses of each buffer copied (thread 0 or
+  // kRowThread, with a barrier between their turns) and consumed (thread 0) so far (a buffer's barriers complete one phase per use)
   __shared__ unsigned s_iss[kRing], s_con[kRing];
   __shared__ uint32_t s_tmem;
   __shared__ int s_li, s_err, s_bb[4];
@@ -491,6 +500,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
   const int count = *p.list_count;
   const int tiles = p.tiles_u * p.tiles_v;
   const int keep = p.keep;
+  const uint32_t idesc = idesc_of(p.ny);
 
   for (;;) {
     __syncthreads();  // every thread is done with the previous grain's shared state
@@ -521,7 +531,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
       s_cs[tid] = cs;
       s_csf[tid] = make_float2((float)cs.x, (float)cs.y);
     }
-    const Geom G = geom_of(p.half[gi], RING);
+    const Geom G = geom_of(p.half[gi], RING, p.nx, p.ny);
     const float mean0 = (float)g.mean0[gi];
     const float c00_rsqrt = g.c0c0[gi] > 0.0 ? (float)(1.0 / sqrt(g.c0c0[gi])) : 0.0f;
     const int gdx = (int)round(g.dx[gi]), gdy = (int)round(g.dy[gi]);
@@ -531,12 +541,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
     if (tid < 2 * G.fw) s_rng[tid] = reinterpret_cast<const unsigned char*>(slotM + wrows)[tid];
     const CUtensorMap* tmap = p.tmaps + gi;  // this grain's operand rows, rotation slots zero-filled to 32
     const CUtensorMap* fmap = p.frame_tmaps + (G.hb >> 1);  // the frame's map for this Hankel width
-    if (tid == 0) {
+    if (tid == 0 || tid == kRowThread)
       asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmap) : "memory");
-      asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(fmap) : "memory");
-    }
+    if (tid == 0) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(fmap) : "memory");
     // ring buffer k: W row at k * 2 wb * 512, M row wb * 512 after it
-    const size_t hbytes = (size_t)(G.rs + 31) * G.hb * 128;
+    const size_t hbytes = (size_t)(G.rs + p.ny - 1) * G.hb * 128;
     unsigned char* sA = smem;
     unsigned char* sHa = sA + (size_t)G.nb * 2 * G.wb * 512;
     unsigned char* sHs = sHa + hbytes;
@@ -624,7 +633,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
       const int nwin = 8 * G.hb;
       const int Xa = Xi & ~7, xoff = Xi - Xa;
       auto stage_rows_at = [&](int xa, int yi, int ys_) {  // thread 0
-        const int boxes = (min(G.rs, G.fw - ys_) + 31 + kStageBoxRows - 1) / kStageBoxRows;
+        const int boxes = (min(G.rs, G.fw - ys_) + p.ny - 1 + kStageBoxRows - 1) / kStageBoxRows;
         const uint32_t sb = smem_u32(&s_stage);
         mbar_expect_tx(sb, (uint32_t)(boxes * kStageBoxRows * G.rp));
         for (int j = 0; j < boxes; ++j)
@@ -641,12 +650,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
           atomicOr(p.error, 1);
         }
       };
-      // Operand rows stream through the ring (thread 0): row y of the tile goes
-      // to buffer y % nb; its copy waits for the MMAs of the row that used the
-      // buffer before (nb rows earlier), and is issued nb - 1 rows ahead of its
-      // MMAs, so the copies overlap the fills and MMAs.
+      // Operand rows stream through the ring: row y of the tile goes to buffer
+      // y % nb; its copy waits for the MMAs of the row that used the buffer
+      // before (nb rows earlier), and is issued nb - 1 rows ahead of its MMAs, so
+      // the copies overlap the fills and MMAs.  Thread 0 issues a tile's first
+      // rows, thread kRowThread the others during the MMA phases, so that the
+      // thread that issues the MMAs does not wait for the previous row's.
       const int NB = G.nb;
-      auto issue_row_of = [&](const CUtensorMap* tm, int y) -> bool {  // thread 0
+      auto issue_row_of = [&](const CUtensorMap* tm, int y) -> bool {  // thread 0 or kRowThread
         const int k = y % NB;
         const unsigned use = s_iss[k];
         if (use > 0 && !mbar_wait(smem_u32(&s_free[k]), (use - 1) & 1u)) return false;
@@ -677,13 +688,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
         if (tid == 0 && s_stage_out) wait_rows();  // this strip's rows (staged during the previous MMAs)
         __syncthreads();
         if (s_err) break;
-        // Hankel image rows ys .. ys + nr + 30 of I - m and of (I - m)^2.
+        // Hankel image rows ys .. ys + nr + ny - 2 of I - m and of (I - m)^2.
         // Entry (block a, shift s) of a row is the 8-pixel window starting at
         // column x = 8 a + s, stored at byte 16 x: a warp fills one row, 25
         // windows per pass, lane x reading pixel x and taking pixels
         // x + 1 .. x + 7 from the next lanes, so the 16-byte stores of a pass
         // are contiguous.  The pixels come from the staged rows.
-        for (int rho = warp; rho < nr + 31; rho += kWarps) {
+        for (int rho = warp; rho < nr + p.ny - 1; rho += kWarps) {
           const uint16_t* srow = reinterpret_cast<const uint16_t*>(sR + (size_t)rho * G.rp) + xoff;
           unsigned char* drow = sHa + (size_t)rho * G.hb * 128;
           unsigned char* qrow = sHs + (size_t)rho * G.hb * 128;
@@ -711,10 +722,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
         if (tid == 0 && !s_err && ys + G.rs < G.fw) stage_rows(ys + G.rs);
         bool committed = false;  // thread 0: MMAs of this strip committed to s_mbar
         if (tid == 0 && !s_err) {
+          // The operands' descriptors advance by additions to their address field
+          // (in 16-byte units): an MMA is issued every dozen instructions, less
+          // than it takes to run even at N = 16.
+          const uint64_t a0 = make_desc(abase, 512, 128), b0 = make_desc(habase, 128, (uint32_t)(G.hb * 128));
+          const uint32_t m_ofs = (uint32_t)(G.wb * 512) >> 4, s_ofs = (hsbase - habase) >> 4;
           for (int yl = 0; yl < nr; ++yl) {
             const int y = ys + yl;
             const int k = y % NB;
             const unsigned use = s_con[k];
+            // chunk c reads footprint blocks 2c - 3 + j, 2c - 2 + j for x shift j: over
+            // the shifts in use, j >= 4 - nx, the chunks touching the row's occupied
+            // blocks [lo, hi] (the others add zeros)
+            const int lo = s_rng[2 * y], hi = s_rng[2 * y + 1];
+            const int c0 = lo >> 1, c1 = min(G.nch - 1, (hi + p.nx - 1) >> 1);
+            uint64_t ad = a0 + ((uint32_t)(k * 2 * G.wb * 512 + c0 * 1024) >> 4);
+            uint64_t bd = b0 + ((uint32_t)((yl * G.hb + 2 * c0) * 128) >> 4);
             if (!mbar_wait(smem_u32(&s_full[k]), use & 1u)) {
               s_err = 1;
               atomicOr(p.error, 1);
@@ -722,30 +745,24 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
             }
             s_con[k] = use + 1;
             asm volatile("tcgen05.fence::after_thread_sync;");
-            // chunk c reads footprint blocks 2c - 3 .. 2c + 1 (over the 4 x-shifts):
-            // the chunks touching the row's occupied blocks [lo, hi]
-            const int lo = s_rng[2 * y], hi = s_rng[2 * y + 1];
-            const int c1 = min(G.nch - 1, (hi + 3) >> 1);
-            const uint32_t wrow = abase + (uint32_t)(k * 2 * G.wb * 512), mrow = wrow + (uint32_t)(G.wb * 512);
-            for (int c = lo >> 1; c <= c1; ++c) {
-              const uint32_t ao = (uint32_t)(2 * c * 512);
-              const uint32_t bo = (uint32_t)((yl * G.hb + 2 * c) * 128);
-              mma_bf16(tmem, make_desc(wrow + ao, 512, 128), make_desc(habase + bo, 128, (uint32_t)(G.hb * 128)),
-                       acc);
-              mma_bf16(tmem + 256u, make_desc(mrow + ao, 512, 128),
-                       make_desc(hsbase + bo, 128, (uint32_t)(G.hb * 128)), acc);
+            for (int c = c0; c <= c1; ++c, ad += 1024 >> 4, bd += 256 >> 4) {
+              mma_bf16(tmem, ad, bd, idesc, acc);
+              mma_bf16(tmem + 256u, ad + m_ofs, bd + s_ofs, idesc, acc);
               acc = 1u;
             }
             mma_commit(smem_u32(&s_free[k]));
-            if (y + NB - 1 < G.fw && !issue_row(y + NB - 1)) {
-              s_err = 1;
-              atomicOr(p.error, 1);
-              break;
-            }
           }
           // also after an error: the MMAs issued before it are then tracked by this phase
           mma_commit(mbar);
           committed = true;
+        }
+        if (tid == kRowThread && !s_err) {
+          for (int y = ys + NB - 1; y < min(ys + nr + NB - 1, G.fw); ++y)
+            if (!issue_row(y)) {
+              s_err = 1;
+              atomicOr(p.error, 1);
+              break;
+            }
         }
         // one thread waits for the MMAs; the others rest at the barrier
         if (tid == 0 && committed) {
@@ -802,6 +819,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
       float sc[2];
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {
+        sc[ch] = -INFINITY;
+        if (q < 4 - p.nx || 8 * h + 4 * ch >= p.ny) continue;  // (warp-uniform: a shift or y offsets outside the zone)
         uint32_t dv[32], sv[32];
         const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * h + 32 * ch);
         tmem_ld32(ta, dv);
