@@ -35,14 +35,11 @@
 
 namespace ptk {
 
-// One step of the walk: with `run`, the map c from distances to `from` (the low
-// word of the bits of an approximate sum) to distances to `to`; then n terms
-// from index `at`; then step next / 2 (negative: the last one).  run = next & 1.
+// One step of the walk: the map k[0], k[1] of the sum's bit pattern, then n
+// terms from index `at`, then step `next` (negative: it was the last one).
 struct __align__(16) SeqStep {
-  int c0, c1, at, n;
-  long long to;
-  unsigned from;
-  int next;
+  long long k0, k1;
+  int at, n, next, pad;
 };
 
 template <int NT>
@@ -82,8 +79,13 @@ __device__ __forceinline__ SeqPlan seq_plan(int P, int G) {
   return SeqPlan{l, P / (1 + 4 * l)};
 }
 
-// NS = 1 or 2 sums of P terms; with two, each takes half of the block's warps
-// (plan: seq_plan(P, NT / NS)).  terms.of(n) provides sum n's terms as a
+// Threads of a block that form one of NS sums side by side: all of its share, up
+// to 128 (more threads shorten the chunks less than they lengthen the scan).
+template <int NT, int NS>
+constexpr int kSeqThreads = NT / NS < 128 ? NT / NS : 128;
+
+// NS = 1 or 2 sums of P terms, each by kSeqThreads<NT, NS> threads (plan:
+// seq_plan(P, kSeqThreads<NT, NS>)).  terms.of(n) provides sum n's terms as a
 // function of their index, which may be asked for up to three terms past the
 // last one (any value will do).  The sums are in seq_scratch<NT>().out once the
 // block has synchronised (the caller does).  Every thread must call it; the
@@ -91,14 +93,14 @@ __device__ __forceinline__ SeqPlan seq_plan(int P, int G) {
 template <int NT, int NS, class Terms>
 __device__ __forceinline__ void seq_sums(int P, const SeqPlan plan, const Terms& terms) {
   static_assert((NS == 1 || NS == 2) && NT % (32 * NS) == 0, "whole warps per sum");
-  constexpr int G = NT / NS;  // threads of one sum
+  constexpr int G = kSeqThreads<NT, NS>;  // threads of one sum
   SeqSumScratch<NT>& sc = seq_scratch<NT>();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n = warp / (G / 32), tid = threadIdx.x - n * G, warp0 = n * (G / 32);
   const auto term = terms.of(n);
   const int l = plan.l, L = 1 + 4 * l, full = plan.full;
   const int beg = tid * L;
-  const bool mine = tid < full;
+  const bool mine = n < NS && tid < full;
   double S[4], A[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) S[u] = A[u] = 0.0;
@@ -130,7 +132,7 @@ __device__ __forceinline__ void seq_sums(int P, const SeqPlan plan, const Terms&
   }
   const double before_me = __shfl_up_sync(0xffffffffu, inc, 1);
   __syncthreads();
-  if (32 * (warp - warp0) < full) {  // (warp-uniform)
+  if (n < NS && 32 * (warp - warp0) < full) {  // (warp-uniform)
     double base = 0.0;
     float total = 0.0f;
 #pragma unroll
@@ -235,60 +237,53 @@ __device__ __forceinline__ void seq_sums(int P, const SeqPlan plan, const Terms&
       }
     }
     const int p0 = __shfl_up_sync(0xffffffffu, c0, 1), p1 = __shfl_up_sync(0xffffffffu, c1, 1);
-    const unsigned from_lo = (unsigned)__double2loint(from) & ~1u;
-    const unsigned first_lo = __shfl_sync(0xffffffffu, from_lo, first), own_lo = __shfl_sync(0xffffffffu, from_lo, own);
+    const long long from_bits = __double_as_longlong(from) & ~1ll;
+    const long long first_bits = __shfl_sync(0xffffffffu, from_bits, first);
+    const long long own_bits = __shfl_sync(0xffffffffu, from_bits, own);
     const int slot = 33 * warp;
+    // In a run the sum's bits change by `to - from`, the approximate sums at its
+    // ends, and by the map of the distances; a run without terms that count
+    // changes nothing.
     if (cnt != 0) {
-      SeqStep e;
-      seq_compose(lane > 0 ? p0 : 0, lane > 0 ? p1 : 0, b0, b1, &e.c0, &e.c1);
-      e.at = at;
-      e.n = cnt;
-      e.to = __double_as_longlong(to) & ~1ll;
-      e.from = lane > 0 ? first_lo : (unsigned)__double2loint(a[0]) & ~1u;
+      int m0, m1;
+      seq_compose(lane > 0 ? p0 : 0, lane > 0 ? p1 : 0, b0, b1, &m0, &m1);
+      const bool run = (b_some | (unsigned)((any & ((1u << lane) - 1u) & ~((1u << first) - 1u)) != 0u)) != 0u;
+      const long long by = (__double_as_longlong(to) & ~1ll) - (lane > 0 ? first_bits : __double_as_longlong(a[0]) & ~1ll);
       const int k = slot + __popc(below);
-      e.next = 2 * (k + 1) + (int)(b_some | (unsigned)((any & ((1u << lane) - 1u) & ~((1u << first) - 1u)) != 0u));
-      sc.list[k] = e;
+      sc.list[k] = SeqStep{run ? by + m0 : 0, run ? by + m1 : 0, at, cnt, k + 1, 0};
     }
     if (lane == 31) {  // the warp's last map, and what the full chunks leave of the terms
       const bool last = 32 * (warp - warp0 + 1) >= full;
-      SeqStep e;
-      e.c0 = c0;
-      e.c1 = c1;
-      e.at = full * L;
-      e.n = last ? P - full * L : 0;
-      e.to = __double_as_longlong(a[4]) & ~1ll;
-      e.from = own_lo;
-      e.next = (last ? -2 : 2 * (slot + 33)) + (int)((any & ~((1u << own) - 1u)) != 0u);
-      sc.list[slot + __popc(cut)] = e;
+      const bool run = (any & ~((1u << own) - 1u)) != 0u;
+      const long long by = (__double_as_longlong(a[4]) & ~1ll) - own_bits;
+      sc.list[slot + __popc(cut)] = SeqStep{run ? by + c0 : 0, run ? by + c1 : 0, full * L, last ? P - full * L : 0,
+                                            last ? -1 : slot + 33, 0};
     }
   }
   __syncthreads();
-  if (tid == 0) {
+  if (n < NS && tid == 0) {
     // The walk of sum n, four terms at a time (past a step's end: + 0, which
     // changes nothing: s is never -0).  Branches cost more than what they would
     // skip here: there is one, the loop's.
     SeqStep e = sc.list[33 * warp];
-    if (full == 0) e = SeqStep{0, 0, 0, P, 0, 0u, -2};  // fewer terms than one chunk
+    if (full == 0) e = SeqStep{0, 0, 0, P, -1, 0};  // fewer terms than one chunk
     double s = 0.0, t[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) t[u] = term(e.at + u);
     bool more;
     do {
-      const SeqStep f = sc.list[max(e.next, 0) >> 1];
-      const int d = __double2loint(s) - (int)e.from;
-      const long long r = e.to + (d + ((d & 1) ? e.c1 : e.c0));
-      s = (e.next & 1) ? __longlong_as_double(r) : s;
+      const SeqStep f = sc.list[max(e.next, 0)];
+      const long long b = __double_as_longlong(s);
+      s = __longlong_as_double(b + ((b & 1) ? e.k1 : e.k0));
 #pragma unroll
       for (int u = 0; u < 4; ++u) s += u < e.n ? t[u] : 0.0;
       const bool rest = e.n > 4;
       more = rest || e.next >= 0;
       e.at = rest ? e.at + 4 : f.at;
       e.n = rest ? e.n - 4 : f.n;
-      e.next = rest ? e.next & ~1 : f.next;
-      e.c0 = f.c0;
-      e.c1 = f.c1;
-      e.to = f.to;
-      e.from = f.from;
+      e.next = rest ? e.next : f.next;
+      e.k0 = rest ? 0 : f.k0;
+      e.k1 = rest ? 0 : f.k1;
 #pragma unroll
       for (int u = 0; u < 4; ++u) t[u] = term(e.at + u);
     } while (more);

@@ -169,16 +169,8 @@ struct ObjGrain {
   double mean0, c0c0;
 };
 
-// Exact integer -> double without the conversion pipe (a sixteenth of the
-// FP64 rate): the bits of 2^52 + v, minus 2^52.
+// exact uint16 -> double without the conversion pipe: the bits of 2^52 + v, minus 2^52
 __device__ __forceinline__ double u16d(unsigned v) { return __hiloint2double(0x43300000, (int)v) - 0x1p52; }
-__device__ __forceinline__ double s32d(int v) {
-  return __hiloint2double(0x43300000, (int)((unsigned)v + 0x80000000u)) - (0x1p52 + 0x1p31);
-}
-// v / 2, exactly
-__device__ __forceinline__ double half_s32d(int v) {
-  return __hiloint2double(0x43200000, (int)((unsigned)v + 0x80000000u)) - (0x1p51 + 0x1p30);
-}
 
 // floor(x) and x - floor(x), both exact, for 0 <= x < 2^31: the nearest
 // integer in the low mantissa bits of x + 1.5 * 2^52, one less where it lies
@@ -191,14 +183,21 @@ __device__ __forceinline__ double split(double x, int* ix) {
   return f + __hiloint2double(below ? 0x3ff00000 : 0, 0);
 }
 
-// cubic1 of four pixels at x (x2 = x * x): its coefficients are multiples of
-// 1/2 below 2^20, which cubic1's operations reach without rounding, so they
-// are formed as integers.
-__device__ __forceinline__ double cubic_px(int p0, int p1, int p2, int p3, double x, double x2) {
-  const double a = half_s32d(3 * (p1 - p2) + p3 - p0);
-  const double b = half_s32d(2 * p0 - 5 * p1 + 4 * p2 - p3);
-  const double c = half_s32d(p2 - p0);
-  return a * x2 * x + b * x2 + c * x + u16d((unsigned)p1);
+// Twice cubic1 of four pixels at x (x2 = x * x): its coefficients are multiples
+// of 1/2 below 2^20, which cubic1's operations reach without rounding, so they
+// are formed as integers, doubled; twice every later operation's value is that
+// operation on doubled values.  The conversions run on their own pipe, at an
+// eighth of the FP64 rate but in one instruction each: with 18 a point, their
+// pipe is as busy as the FP64 one.  (Through the bits of 2^52 + v, which takes
+// three instructions, an evaluation issued 397 instructions per warp and point
+// in all, 122 of them FP64, instead of 357 and 105: 400 grains 7.77 -> 7.63 ms,
+// 2000 27.2 -> 26.5 ms.)
+__device__ __forceinline__ double cubic_px_twice(int p0, int p1, int p2, int p3, double x, double x2) {
+  const int d = p1 - p2, t = p3 - p0;
+  const double a = (double)(3 * d + t);
+  const double b = (double)(p0 - p1 - t - 4 * d);
+  const double c = (double)(p2 - p0);
+  return __fma_rn(2.0, (double)p1, a * x2 * x + b * x2 + c * x);
 }
 
 // cubic1 with its multiplications by 2 and 1/2 folded: they are exact, so a
@@ -231,6 +230,8 @@ struct ExactObj {
   int v_at, d0_at;     // bytes from the start of the dynamic shared memory
   int clamped;
   double rot, c1, s1;  // the last rotation angle, its cosine and sine
+  double X[3];         // the point to evaluate next
+  int done;            // no further one
 };
 __device__ __forceinline__ ExactObj& exact_obj() {
   __shared__ ExactObj s;
@@ -320,7 +321,7 @@ __device__ __forceinline__ void sample_staged(const ExactObj& ex, double xpix1, 
     const uint16_t* px[kAt];
 #pragma unroll
     for (int k = 0; k < kAt; ++k) {
-      const double x = s32d(q[k].x), y = s32d(q[k].y);
+      const double x = (double)q[k].x, y = (double)q[k].y;
       const double xs = xpix1 + c1 * x + s1 * y;
       const double ys = ypix1 - s1 * x + c1 * y;
       int ix, iy;
@@ -341,8 +342,9 @@ __device__ __forceinline__ void sample_staged(const ExactObj& ex, double xpix1, 
         const double y2 = y01[k] * y01[k];
         double arr[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) arr[j] = cubic_px(p[j], p[w + j], p[2 * w + j], p[3 * w + j], y01[k], y2);
-        val[k] = cubic1_fast(arr[0], arr[1], arr[2], arr[3], x01[k]);
+        for (int j = 0; j < 4; ++j)
+          arr[j] = cubic_px_twice(p[j], p[w + j], p[2 * w + j], p[3 * w + j], y01[k], y2);
+        val[k] = 0.5 * cubic1_fast(arr[0], arr[1], arr[2], arr[3], x01[k]);
       } else {
         double arr[4];
 #pragma unroll
@@ -362,18 +364,18 @@ __device__ __forceinline__ void sample_staged(const ExactObj& ex, double xpix1, 
 // reference's operations and order, every product and sum rounded separately
 // (this file is compiled without FMA contraction), cos / sin correctly
 // rounded (ptk_crtrig.cuh) where the host C library is within an ulp.  The
-// block's threads interpolate the points in parallel into shared memory (82 FP64
-// operations a point, none of them a conversion, which runs at an eighth of
-// their rate: 206 operations' time before), then form the sums of the reference's two loops over them,
+// block's threads interpolate the points in parallel into shared memory (66 FP64
+// operations a point, and 18 conversions on their own pipe), then form the sums of the reference's two loops over them,
 //     mean1 = (sum v) * (1 / P),  C0C1 = sum d0 (v - mean1),  C1C1 = sum (v - mean1)^2
 // (d0 = I0 - mean0), each rounded after every point in point order as those
 // loops round it (seq_sums), so that the value is the reference's bit for bit
 // and Powell takes the reference's path even where the objective is flat.
-// Called by every thread of the block with the same X; returns the same value
-// on every thread.  Not inlined: Powell calls it from a dozen places.
+// Called by every thread of the block, with X in exact_obj().X; the value is the
+// first warp's return.  Not inlined: Powell calls it from a dozen places.
 template <int NT, class Ref>
-__device__ __noinline__ double objective_exact(double X0, double X1, double X2) {
+__device__ __noinline__ double objective_exact() {
   ExactObj& ex = exact_obj();
+  const double X0 = ex.X[0], X1 = ex.X[1], X2 = ex.X[2];
   const int tid = threadIdx.x;
   const double xpix1 = ex.xref + X0;
   const double ypix1 = ex.yref + X1;
@@ -420,6 +422,7 @@ __device__ __noinline__ double objective_exact(double X0, double X1, double X2) 
   __syncthreads();
   seq_sums<NT, 2>(ex.P, ex.two, SumC<Ref>{obj_v(ex), Ref(ex)});
   __syncthreads();
+  if (tid >= 32) return 0.0;
   const double ncc = sc.out[0] / sqrt(ex.c0c0 * sc.out[1]);
   double W = 1.0;
   const double d2 = X0 * X0 + X1 * X1;
@@ -447,8 +450,8 @@ __device__ __forceinline__ void exact_begin(const ObjGrain& o, const GrainsDev& 
     ex.cur = cur;
     ex.interp = sp.interp;
     ex.P = o.P;
-    ex.one = seq_plan(o.P, NT);
-    ex.two = seq_plan(o.P, NT / 2);
+    ex.one = seq_plan(o.P, kSeqThreads<NT, 1>);
+    ex.two = seq_plan(o.P, kSeqThreads<NT, 2>);
     ex.xref = o.xref;
     ex.yref = o.yref;
     ex.drot = o.drot;
@@ -463,6 +466,7 @@ __device__ __forceinline__ void exact_begin(const ObjGrain& o, const GrainsDev& 
     ex.v_at = v_at;
     ex.d0_at = d0_at;
     ex.clamped = 0;
+    ex.done = 0;
     ex.rot = __longlong_as_double(0x7ff8000000000000ll);
   }
   __syncthreads();
@@ -553,10 +557,16 @@ __device__ ObjGrain load_grain(const GrainsDev& g, int gi) {
 }
 
 // --- Powell on the device, block-uniform ----------------------------------
+// The first warp runs Powell, the others take part in its evaluations only (the
+// minimiser's scalar FP64 work, repeated by every warp, would compete with the
+// samples of the other blocks on the SM).
 template <int NT, class Ref>
 struct PowellEval {
   __device__ __forceinline__ double operator()(const double X[3]) const {
-    return objective_exact<NT, Ref>(X[0], X[1], X[2]);
+    ExactObj& ex = exact_obj();
+    if (threadIdx.x < 3) ex.X[threadIdx.x] = threadIdx.x == 0 ? X[0] : (threadIdx.x == 1 ? X[1] : X[2]);
+    __syncthreads();
+    return objective_exact<NT, Ref>();
   }
 };
 
@@ -739,12 +749,12 @@ constexpr int kPatchMargin = 6;
 // follow_pattern_subpixel_xyR (src/p-tracker.cpp:1090-1128) for every grain,
 // one block per grain, grains taken in `order` (decreasing pattern size) when
 // given.  A grain takes 160-400 evaluations one after another, so an
-// evaluation's latency counts: for 441 points 11.8k cycles (2.0k samples, 3.4k
-// the first sum, 4.7k the other two, 0.4k cosine and sine, 1.3k Powell's own
+// evaluation's latency counts: for 441 points 11.5k cycles (2.0k samples, 3.4k
+// the first sum, 4.5k the other two, 0.4k cosine and sine, 1.3k Powell's own
 // divisions and roots), against 33k with the sums and the cosine's series in one
-// thread.  Of whole pairs: 12 grains of up to 530 points 3.57 -> 1.95 ms, 400 of
-// 1,260-2,820 (8-bit frames of 2048x1536) 20.5 -> 7.7 ms, 2000 of up to 5,025
-// (5616x3744) 47.7 -> 27.2 ms of which the search takes 9.4.
+// thread.  Of whole pairs: 12 grains of up to 530 points 3.57 -> 1.83 ms, 400 of
+// 1,260-2,820 (8-bit frames of 2048x1536) 20.5 -> 7.6 ms, 2000 of up to 5,025
+// (5616x3744) 47.7 -> 26.5 ms of which the search takes 9.2.
 template <int NT, int BLOCKS, class Ref>
 __global__ void __launch_bounds__(NT, BLOCKS) k_subpix_powell(GrainsDev g, FrameDev cur, SubpixParams sp,
                                                               int patch_cap, int max_points, const int* order,
@@ -778,11 +788,20 @@ __global__ void __launch_bounds__(NT, BLOCKS) k_subpix_powell(GrainsDev g, Frame
     s_patch[e] = cur.pix[(size_t)(py0 + yy) * cur.pitch + (px0 + xx)];
   }
   exact_begin<NT, Ref>(o, g, cur, sp, reach, px0, py0, pw, ph, v_at, d0_at);
+  ExactObj& ex = exact_obj();
+  if (threadIdx.x >= 32) {
+    for (;;) {
+      __syncthreads();
+      if (ex.done) return;
+      objective_exact<NT, Ref>();
+    }
+  }
   const PowellEval<NT, Ref> f{};
   double X[3] = {0.0, 0.0, 0.0};
   double fret;
   powell_minimize(f, X, sp.init_dir, sp.tol, &fret);
   if (threadIdx.x == 0) {
+    ex.done = 1;
     g.ncc_subpix[gi] = 1.0 - fret;
     g.upix[gi] += X[0];
     g.vpix[gi] += X[1];
@@ -790,8 +809,9 @@ __global__ void __launch_bounds__(NT, BLOCKS) k_subpix_powell(GrainsDev g, Frame
     g.dx[gi] += X[0];
     g.dy[gi] += X[1];
     g.drot[gi] += X[2];
-    if (exact_obj().clamped) g.status[gi] |= PTK_ST_SUBPIX_CLAMPED;
+    if (ex.clamped) g.status[gi] |= PTK_ST_SUBPIX_CLAMPED;
   }
+  __syncthreads();  // lets the other warps go
 }
 
 // Objective at caller-given X for every grain, as Powell evaluates it.
@@ -805,7 +825,9 @@ __global__ void __launch_bounds__(kSubpixThreads) k_objective(GrainsDev g, Frame
   }
   // one evaluation: no frame region is staged
   exact_begin<kSubpixThreads, RefGlobal>(o, g, cur, sp, 0, 0, 0, 0, 0, 0, 0);
-  const double val = objective_exact<kSubpixThreads, RefGlobal>(Xall[3 * gi], Xall[3 * gi + 1], Xall[3 * gi + 2]);
+  if (threadIdx.x < 3) exact_obj().X[threadIdx.x] = Xall[3 * gi + threadIdx.x];
+  __syncthreads();
+  const double val = objective_exact<kSubpixThreads, RefGlobal>();
   if (threadIdx.x == 0) f[gi] = val;
 }
 
@@ -856,7 +878,8 @@ static bool powell_staged(int max_points) { return (size_t)max_points * 2 * size
 // grains than SMs (each block has an SM to itself, and its evaluations'
 // latency is the whole time) and patterns large enough to keep 256 busy: 80
 // grains of up to 5,000 points 18.9 -> 17.4 ms, 40 of up to 2,100 equal, 12 of
-// up to 530 1.88 -> 2.11 ms, 2000 grains of up to 5,000 27.4 -> 28.9 ms.
+// up to 530 1.88 -> 2.03 ms, 400 of up to 2,820 7.8 -> 8.6 ms, 2000 of up to
+// 5,000 27.2 -> 28.4 ms.
 constexpr int kPowellWidePoints = 1500;
 typedef void (*PowellKernel)(GrainsDev, FrameDev, SubpixParams, int, int, const int*, const int*);
 static PowellKernel powell_kernel(int n, int max_points, int num_sms, int* threads) {
