@@ -615,6 +615,8 @@ int enqueue_search(ptk_ctx* c, int level, cudaStream_t s, cudaEvent_t* ev = null
     b.tiles_v = sg.tiles_v;
     b.nx = std::min(4, (sg.nu + 7) / 8);
     b.ny = std::min(kTileV, (sg.nv + 1) & ~1);
+    b.num_sms = c->num_sms;
+    b.wsplit = bf16_weight_splits(c->n, sg.nrot, c->num_sms);
     b.keep = std::min(std::max(c->cfg.topk, 1), kBf16KeepMax);
     b.max_items = (int)sg.items;
     b.half = c->d_bf_half;

@@ -98,6 +98,7 @@ struct FinalizeLaunch {
 
 // BF16 tensor-core search: kept candidates per tile (upper bound of `keep`).
 constexpr int kBf16KeepMax = 8;
+constexpr int kBf16WeightSplits = 8;
 constexpr int kBf16FrameMaps = 9;  // frame tensor maps per frame buffer, one per Hankel width
 
 struct Bf16Launch {
@@ -111,8 +112,10 @@ struct Bf16Launch {
   int left, right, up, down;
   int tiles_u, tiles_v;
   int nx, ny;               // a tile's 8-column x shifts (1..4) and y offsets (even, 2..32) that any of the zone's tiles needs
+  int wsplit;               // blocks of a grain's weights, each with its share of the rotation steps (1..kBf16WeightSplits)
   int keep;                 // candidates per tile rescored exactly (1..kBf16KeepMax)
   int max_items;            // list capacity x tiles: grid of the per-tile kernels
+  int num_sms;
   const int* half;          // per grain: footprint half-extent ceil(max |offset|) + 1
   const size_t* wofs;       // per grain: offset of its weight slot in wslots (16-byte units)
   unsigned char* wslots;    // BF16 weights of the level's rotation steps, per grain
@@ -173,6 +176,7 @@ bool bf16_supported(int max_r, int nrot, int max_dup);
 bool bf16_ring_ok(int max_half, int ring);
 constexpr int kBf16RingDefault = 4;
 size_t bf16_weight_entries(int half);
+int bf16_weight_splits(int n, int nrot, int num_sms);
 bool bf16_encode_tmaps(const int* half, const size_t* wofs, int n, unsigned char* wslots, int nrot,
                        CUtensorMap* out);
 bool bf16_encode_frame_tmaps(const uint16_t* pix, int dimx, int dimy, int pitch, CUtensorMap* out);

@@ -78,6 +78,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <climits>
 #include <mutex>
 
@@ -291,7 +292,8 @@ __device__ __forceinline__ bool better_b(double ncc, int idx, double bn, int bi)
 //    (high 8 bits), with integer shared-memory atomics.  Written to the
 //    grain's slot as W_r = sum I0 - count * mean0 and M_r = count, each
 //    [footprint row][8-column block][rotation][8 values], M after W.  As many
-//    rotations per pass as maps fit in shared memory.
+//    rotations per pass as maps fit in shared memory; with few grains, several
+//    blocks per grain, each with its share of the rotations.
 __global__ void __launch_bounds__(kWThreads) k_weights_bf16(Bf16Launch p) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double2 s_cs[kNRot];
@@ -315,7 +317,9 @@ __global__ void __launch_bounds__(kWThreads) k_weights_bf16(Bf16Launch p) {
   __shared__ unsigned char s_occ[kMaxFoot * 12];  // [row][8-column block]: a point in some rotation step
   for (int e = tid; e < rows; e += kWThreads) s_occ[e] = 0;
   const double base_rot = g.refrot[gi] + g.drot[gi];  // total_rot = base_rot + step, as the exact search
-  if (tid < p.nrot) {
+  const int share = (p.nrot + p.wsplit - 1) / p.wsplit;  // (no share is empty: bf16_weight_splits)
+  const int r_beg = blockIdx.y * share, r_end = min(r_beg + share, p.nrot);
+  if (tid >= r_beg && tid < r_end) {
     double sr, cr;
     sincos(base_rot + p.steps[tid], &sr, &cr);
     s_cs[tid] = make_double2(cr, sr);
@@ -327,10 +331,10 @@ __global__ void __launch_bounds__(kWThreads) k_weights_bf16(Bf16Launch p) {
   // per rotation step a map of fw rows of fwp = 8 nbf words (the columns past
   // fw stay zero), so that a block's 8 words are two 16-byte loads
   const int fwp = 8 * G.nbf, fw2 = G.fw * fwp;
-  const int nb_max = max(1, min(p.nrot, kWSmem / (4 * fw2)));
+  const int nb_max = max(1, min(r_end - r_beg, kWSmem / (4 * fw2)));
   unsigned* map = reinterpret_cast<unsigned*>(smem);
-  for (int r0 = 0; r0 < p.nrot; r0 += nb_max) {
-    const int nb = min(nb_max, p.nrot - r0);
+  for (int r0 = r_beg; r0 < r_end; r0 += nb_max) {
+    const int nb = min(nb_max, r_end - r0);
     for (int e = tid; e < nb * fw2 / 4; e += kWThreads) reinterpret_cast<uint4*>(map)[e] = make_uint4(0, 0, 0, 0);
     __syncthreads();
     // four points per thread at a time: their loads are in flight together
@@ -410,8 +414,8 @@ __global__ void __launch_bounds__(kWThreads) k_weights_bf16(Bf16Launch p) {
     __syncthreads();
   }
   // per footprint row: the first and last 8-column block holding a point of
-  // any rotation step (an empty row: first > last)
-  unsigned char* rng = reinterpret_cast<unsigned char*>(slotM + (size_t)rows * p.nrot);
+  // any of this block's rotation steps (an empty row: first > last)
+  unsigned char* rng = reinterpret_cast<unsigned char*>(slotM + (size_t)rows * p.nrot) + 2 * G.fw * blockIdx.y;
   if (tid < G.fw) {
     int lo = 255, hi = 0;
     for (int a = G.nbf - 1; a >= 0; --a)
@@ -538,7 +542,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
     const size_t wrows = (size_t)G.fw * G.nbf * p.nrot;
     const uint4* slotW = reinterpret_cast<const uint4*>(p.wslots) + p.wofs[gi];
     const uint4* slotM = slotW + wrows;
-    if (tid < 2 * G.fw) s_rng[tid] = reinterpret_cast<const unsigned char*>(slotM + wrows)[tid];
+    if (tid < 2 * G.fw) {  // over the blocks that share the rotation steps: the first block's minimum, the last one's maximum
+      const unsigned char* rng = reinterpret_cast<const unsigned char*>(slotM + wrows) + tid;
+      int v = rng[0];
+      for (int k = 1; k < p.wsplit; ++k) v = tid & 1 ? max(v, (int)rng[2 * G.fw * k]) : min(v, (int)rng[2 * G.fw * k]);
+      s_rng[tid] = (unsigned char)v;
+    }
     const CUtensorMap* tmap = p.tmaps + gi;  // this grain's operand rows, rotation slots zero-filled to 32
     const CUtensorMap* fmap = p.frame_tmaps + (G.hb >> 1);  // the frame's map for this Hankel width
     if (tid == 0 || tid == kRowThread)
@@ -985,9 +994,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
 //    weak keep margin below the grain's best tile are not rescored.  One block per (grain, tile); a work unit is one rotation
 //    step for two candidates that both need it (or one), taken by one warp
 //    whose lanes share the pattern points; per candidate the best record over
-//    its rotation steps in the reference's order.
-__global__ void __launch_bounds__(256, 4) k_rescore_bf16(Bf16Launch p) {
-  constexpr int kW = 8;
+//    its rotation steps in the reference's order.  NT threads: a block's units
+//    run side by side in its warps, so with few blocks each gets more of them
+//    (launch_search_bf16).
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_rescore_bf16(Bf16Launch p) {
+  constexpr int kW = NT / 32;
   __shared__ double s_bn[kBf16KeepMax][kW];
   __shared__ int s_bi[kBf16KeepMax][kW];
   __shared__ int s_base[kBf16KeepMax], s_uv[kBf16KeepMax];
@@ -1011,51 +1023,55 @@ __global__ void __launch_bounds__(256, 4) k_rescore_bf16(Bf16Launch p) {
   const int b = g.pstart[gi], P = g.pstart[gi + 1] - b;
   const bool skip = g.masked[gi] || (g.flags[gi] & 7) || P <= 0 || P > kMaxPatternPoints;
   const int NU = p.left + p.right + 1, NV = p.up + p.down + 1;
-  if (tid == 0) {  // the kept candidates, compacted: anchor pixel index and order index without the rotation
-    int nk = 0, nu = 0;
+  if (warp == 0) {  // the kept candidates, compacted: anchor pixel index and order index without the rotation
     // a tile whose best score lies further below the grain's best tile than
     // the weak keep margin cannot hold the exact best (the keep rule's bound)
     bool far = false;
     if (tiles > 1) {
       const float* tt = p.tile_top + (size_t)li * tiles;
       float best = -INFINITY;
-      for (int k = 0; k < tiles; ++k) best = fmaxf(best, tt[k]);
+      for (int k = lane; k < tiles; k += 32) best = fmaxf(best, tt[k]);
+      for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
       far = best > 0.0f && tt[item - li * tiles] < best * (1.0f - kKeepRelWeak);
     }
-    if (!skip && !far) {
-      const int2* cand = p.topk + (size_t)item * kBf16KeepMax;
-      const unsigned* rots = p.topk_rot + (size_t)item * kBf16KeepMax;
-      const int gdx = (int)round(g.dx[gi]), gdy = (int)round(g.dy[gi]);
-      unsigned rm[kBf16KeepMax];
-      for (int k = 0; k < p.keep && k < kBf16KeepMax; ++k) {
-        const int2 c = cand[k];
-        if (c.x == INT_MIN) continue;
-        s_base[nk] = (g.refy[gi] + gdy + c.y) * p.cur.pitch + (g.refx[gi] + gdx + c.x);
-        s_uv[nk] = (c.x + p.left) * NV + (c.y + p.up);
-        rm[nk] = rots[k];
-        ++nk;
-      }
-      // units: per rotation step, the candidates that need it, two at a time
-      for (int r = 0; r < p.nrot; ++r) {
-        int first = -1;
-        for (int k = 0; k < nk; ++k) {
-          if (!((rm[k] >> r) & 1u)) continue;
-          if (first < 0) {
-            first = k;
-          } else {
-            s_unit[nu++] = r | (first << 8) | (k << 16);
-            first = -1;
-          }
-        }
-        if (first >= 0) s_unit[nu++] = r | (first << 8) | (255 << 16);
-      }
+    int2 c = make_int2(INT_MIN, INT_MIN);
+    unsigned rots = 0u;
+    if (!skip && !far && lane < p.keep && lane < kBf16KeepMax) {
+      c = p.topk[(size_t)item * kBf16KeepMax + lane];
+      if (c.x != INT_MIN) rots = p.topk_rot[(size_t)item * kBf16KeepMax + lane];
     }
-    s_nk = nk;
-    s_nu = nu;
+    const unsigned kept = __ballot_sync(0xffffffffu, c.x != INT_MIN);
+    if (c.x != INT_MIN) {
+      const int gdx = (int)round(g.dx[gi]), gdy = (int)round(g.dy[gi]), k = __popc(kept & ((1u << lane) - 1u));
+      s_base[k] = (g.refy[gi] + gdy + c.y) * p.cur.pitch + (g.refx[gi] + gdx + c.x);
+      s_uv[k] = (c.x + p.left) * NV + (c.y + p.up);
+    }
+    // lane r: the candidates that need rotation step r, two at a time a unit
+    unsigned need = 0u;
+    int k = 0;
+    for (unsigned m = kept; m; m &= m - 1u, ++k)
+      need |= ((__shfl_sync(0xffffffffu, rots, __ffs(m) - 1) >> lane) & 1u) << k;
+    if (lane >= p.nrot) need = 0u;
+    const int units = (__popc(need) + 1) >> 1;
+    int at = units;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += y;
+    }
+    if (lane == 31) s_nu = at;
+    at -= units;
+    while (need) {
+      const int first = __ffs(need) - 1;
+      need &= need - 1u;
+      const int second = need ? __ffs(need) - 1 : 255;
+      need &= need - 1u;
+      s_unit[at++] = lane | (first << 8) | (second << 16);
+    }
+    if (lane == 0) s_nk = __popc(kept);
   }
-  if (tid < kBf16KeepMax * kW) {
-    s_bn[tid / kW][tid % kW] = 0.0;
-    s_bi[tid / kW][tid % kW] = INT_MAX;
+  for (int e = tid; e < kBf16KeepMax * kW; e += NT) {
+    s_bn[e / kW][e % kW] = 0.0;
+    s_bi[e / kW][e % kW] = INT_MAX;
   }
   __syncthreads();
   const int nk = s_nk;
@@ -1133,8 +1149,20 @@ __global__ void __launch_bounds__(256, 4) k_rescore_bf16(Bf16Launch p) {
 // ---------------------------------------------------------------------------
 size_t bf16_weight_entries(int half) {
   const Geom G = geom_of(half);
-  // W, M, per-row block ranges (2 fw <= 190 bytes, padded to keep slots 512-byte aligned)
-  return 2 * (size_t)G.fw * G.nbf * kNRot + kNRot;
+  // W, M, per-row block ranges (2 fw <= 190 bytes for each of the grain's
+  // weights blocks, padded to keep slots 512-byte aligned)
+  static_assert(2 * (kMaxFoot - 1) * kBf16WeightSplits <= 3 * kNRot * 16, "block ranges");
+  return 2 * (size_t)G.fw * G.nbf * kNRot + 3 * kNRot;
+}
+
+// Blocks per grain of the weights kernel (two of which run on an SM): with fewer
+// than four grains per SM, as many as fill four blocks per SM, without an
+// empty share.  40 grains 24.7 -> 12.6 us, 400 grains 59.6 -> 56 us; 2000 grains
+// keep one block each.
+int bf16_weight_splits(int n, int nrot, int num_sms) {
+  const int want = std::min({kBf16WeightSplits, nrot, n > 0 ? (4 * num_sms + n - 1) / n : 1});
+  const int share = (nrot + want - 1) / want;
+  return (nrot + share - 1) / share;
 }
 
 // The weights kernel counts the points landing on a pixel in 8 bits: a
@@ -1234,7 +1262,7 @@ bool bf16_encode_frame_tmaps(const uint16_t* pix, int dimx, int dimy, int pitch,
 void launch_search_bf16(const Bf16Launch& p, int grid, cudaStream_t s, cudaEvent_t* ev, cudaEvent_t frame_ready) {
   const int items = p.max_items;
   if (ev) cudaEventRecord(ev[0], s);
-  k_weights_bf16<<<p.max_items / (p.tiles_u * p.tiles_v), kWThreads, kWSmem, s>>>(p);
+  k_weights_bf16<<<dim3(p.max_items / (p.tiles_u * p.tiles_v), p.wsplit), kWThreads, kWSmem, s>>>(p);
   // the weights need only the reference frame: the current one may still be uploading until here
   if (frame_ready) cudaStreamWaitEvent(s, frame_ready, cudaEventWaitExternal);
   if (ev) cudaEventRecord(ev[1], s);
@@ -1245,7 +1273,12 @@ void launch_search_bf16(const Bf16Launch& p, int grid, cudaStream_t s, cudaEvent
     default: k_search_bf16<4><<<grid, kThreads, kSmemBudget, s>>>(p); break;
   }
   if (ev) cudaEventRecord(ev[2], s);
-  k_rescore_bf16<<<items, 256, 0, s>>>(p);
+  // 256 threads a block fill the SMs from four blocks per SM on; with fewer
+  // blocks, wider ones: 40 grains 52 -> 34.8 us (1024 threads), 400 grains 97 ->
+  // 82 us (512); 2000 grains 180 -> 163 us by the units being listed by a warp.
+  if (items <= p.num_sms) k_rescore_bf16<1024><<<items, 1024, 0, s>>>(p);
+  else if (items < 4 * p.num_sms) k_rescore_bf16<512><<<items, 512, 0, s>>>(p);
+  else k_rescore_bf16<256><<<items, 256, 0, s>>>(p);
   if (ev) cudaEventRecord(ev[3], s);
 }
 
