@@ -15,25 +15,11 @@
 // file is compiled with -fmad=false; the cos/sin of the two parallax angles
 // come from the host.  With both, the device repeats the CPU restatement's
 // FP64 operations exactly.
+#include "ptk_cubic.cuh"
 #include "ptk_internal.cuh"
 #include "ptk_undistor.cuh"
 
 namespace ptk {
-
-namespace {
-
-__device__ __forceinline__ double cubic1(double p0, double p1, double p2, double p3, double x) {
-  const double f0 = p1, f1 = p2;
-  const double fp0 = 0.5 * (p2 - p0);
-  const double fp1 = 0.5 * (p3 - p1);
-  const double d = f0, c = fp0;
-  const double b = -3.0 * f0 + 3.0 * f1 - 2.0 * fp0 - fp1;
-  const double a = 2.0 * f0 - 2.0 * f1 + fp0 + fp1;
-  const double x2 = x * x;
-  return (a * x2 * x + b * x2 + c * x + d);
-}
-
-}  // namespace
 
 __global__ void k_remap_build(Disto X, double2* map, int dimx, int dimy) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -59,32 +45,32 @@ __global__ void k_remap_build(Disto X, double2* map, int dimx, int dimy) {
 
 // One output row per blockIdx.y; a thread per output pixel.  The 4x4 support
 // is gathered through the read-only path; rows of neighbouring threads are
-// adjacent, so each warp's 16 loads touch a few cache lines.
+// adjacent, so each warp's 16 loads touch a few cache lines.  Bound by the FP64
+// and conversion pipes (57 and 13 operations a pixel, 120 and 104 cycles a warp;
+// with every pixel and coordinate converted and the coefficients in FP64 about
+// 105 and 23), then by the 22 bytes a pixel: 5616x3744, with the copy back, 248
+// -> 168 us.
 __global__ void k_remap_apply(const double2* __restrict__ map, const uint16_t* __restrict__ src,
                               uint16_t* __restrict__ dst, int pitch, int dimx, int dimy) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y;
   if (x >= dimx || y >= dimy) return;
   const double2 m = map[(size_t)y * dimx + x];
-  const int ix = (int)floor(m.x), iy = (int)floor(m.y);
-  uint16_t out = 0;
-  if (ix >= 1 && iy >= 1 && ix + 2 < dimx && iy + 2 < dimy) {
-    const double x01 = m.x - (double)ix, y01 = m.y - (double)iy;
+  int out = 0;
+  if (m.x >= 1.0 && m.y >= 1.0 && m.x < (double)(dimx - 2) && m.y < (double)(dimy - 2)) {
+    int ix, iy;
+    const double x01 = split(m.x, &ix), y01 = split(m.y, &iy);
+    const double y2 = y01 * y01;
+    const uint16_t* p0 = src + (size_t)(iy - 1) * pitch + (ix - 1);
+    const uint16_t *p1 = p0 + pitch, *p2 = p1 + pitch, *p3 = p2 + pitch;
     double arr[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int xx = ix - 1 + i;
-      const double q0 = (double)__ldg(&src[(size_t)(iy - 1) * pitch + xx]);
-      const double q1 = (double)__ldg(&src[(size_t)iy * pitch + xx]);
-      const double q2 = (double)__ldg(&src[(size_t)(iy + 1) * pitch + xx]);
-      const double q3 = (double)__ldg(&src[(size_t)(iy + 2) * pitch + xx]);
-      arr[i] = cubic1(q0, q1, q2, q3, y01);
-    }
-    double r = floor(cubic1(arr[0], arr[1], arr[2], arr[3], x01) + 0.5);
-    r = r < 0.0 ? 0.0 : (r > 65535.0 ? 65535.0 : r);
-    out = (uint16_t)r;
+    for (int i = 0; i < 4; ++i)
+      arr[i] = cubic_px_twice(__ldg(p0 + i), __ldg(p1 + i), __ldg(p2 + i), __ldg(p3 + i), y01, y2);
+    const int r = __double2int_rd(__fma_rn(0.5, cubic1_fast(arr[0], arr[1], arr[2], arr[3], x01), 0.5));
+    out = min(max(r, 0), 65535);
   }
-  dst[(size_t)y * pitch + x] = out;
+  dst[(size_t)y * pitch + x] = (uint16_t)out;
 }
 
 void launch_remap_build(const double* params14, const double* trig4, double2* map, int dimx, int dimy,
