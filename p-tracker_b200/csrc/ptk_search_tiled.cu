@@ -21,11 +21,16 @@
 //  * If a column has more runs than the per-column list holds (sparse custom
 //    patterns), the work item computes S1 and S11 entry by entry instead.
 //
-// Thread layout: 256 threads; lane = x offset, warp w = y offsets
-// 8 (w mod 4) .. 8 (w mod 4) + 7 of a 32x32 candidate tile, over the map
-// columns of parity w / 4; the two column halves are summed through shared
-// memory at the end.  The patch pitch is a template constant so every
-// shared-memory address in the inner loop is a register plus an immediate.
+// Thread layout: 256 threads.  A tile of nu x nv candidates has nu * ceil(nv / 8)
+// pairs of an x offset and 8 consecutive y offsets, a pair per lane; they take
+// 1, 2 or 4 warps, and the 8, 4 or 2 classes of warps share the map columns
+// (every 8th, 4th or 2nd), their sums added through shared memory at the end.
+// So a small zone's columns are spread over the warps that a full 32x32 tile
+// needs for its candidates: +-8 (17x17, 2 warps a class), 400 grains of 1,260 to
+// 2,820 points 2.43 -> 1.46 ms; +-6, 40 grains 156 -> 70 us; +-15 (31x31, 4 warps
+// a class as before), 2000 grains 9.23 -> 9.14 ms.  The patch pitch is
+// a template constant so every shared-memory address in the inner loop is a
+// register plus an immediate.
 #include <climits>
 
 #include "ptk_internal.cuh"
@@ -75,7 +80,7 @@ __host__ __device__ inline int tiled_pitch(int max_r) { return 2 * max_r + 1 + k
 __host__ __device__ inline size_t tiled_map_bytes(int max_r) {
   const TiledGeom t = tiled_geom(max_r);
   size_t b = (size_t)t.mw * t.mh * 8;
-  const size_t partial = (size_t)(kTiledThreads / 2) * kTT * 24;  // column-half partial sums
+  const size_t partial = (size_t)kTiledThreads * kTT * 20;  // column-class partial sums
   return b < partial ? partial : b;
 }
 
@@ -105,15 +110,12 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_search_tiled(SearchLaunch 
   int* s_nrun = s_ext + G.mw;
   const size_t pofs = (map_bytes + (size_t)G.mw * kRunsPerCol * 4 + (size_t)G.mw * 8 + 15) & ~(size_t)15;
   uint16_t* s_patch = reinterpret_cast<uint16_t*>(smem + pofs);
-  // partial sums of the second column half reuse the map region after the FMAs
+  // partial sums of all column classes but the first reuse the map region after the FMAs
   double* s_pacc = reinterpret_cast<double*>(smem);
-  unsigned long long* s_p11 = reinterpret_cast<unsigned long long*>(smem + (size_t)(kTiledThreads / 2) * kTT * 8);
-  unsigned* s_p1 = reinterpret_cast<unsigned*>(smem + (size_t)(kTiledThreads / 2) * kTT * 16);
+  unsigned long long* s_p11 = reinterpret_cast<unsigned long long*>(smem + (size_t)kTiledThreads * kTT * 8);
+  unsigned* s_p1 = reinterpret_cast<unsigned*>(smem + (size_t)kTiledThreads * kTT * 16);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int half = warp >> 2;       // column parity handled by this warp
-  const int rb = kTT * (warp & 3);  // first y offset (within the tile) of this thread
-  const int pidx = tid & (kTiledThreads / 2 - 1);
   const int count = *p.list_count;
   const int per_grain = p.nrot * p.tiles_u * p.tiles_v;
   long long total = (long long)count * per_grain;
@@ -178,6 +180,13 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_search_tiled(SearchLaunch 
     const int bw = bx1 - bx0 + 1, bh = by1 - by0 + 1;
     const int u0 = -p.left + tu * kTileU, u1 = min(u0 + kTileU - 1, p.right);
     const int v0 = -p.up + tv * kTileV, v1 = min(v0 + kTileV - 1, p.down);
+    // this thread's candidates: x offset ul, y offsets rb .. rb + 7 of the tile, over
+    // the map columns of class `cls` (of `ncls`)
+    const int nu = u1 - u0 + 1, nvg = (v1 - v0 + kTT) / kTT, pairs = nu * nvg;
+    const int wpc = pairs <= 32 ? 1 : (pairs <= 64 ? 2 : 4), ncls = kTiledThreads / 32 / wpc;
+    const int cls = warp / wpc, pair = (warp - cls * wpc) * 32 + lane;
+    const bool active = pair < pairs;  // (the others repeat the first pair)
+    const int vg = active ? pair / nu : 0, ul = active ? pair - vg * nu : 0, rb = kTT * vg;
     const int X0 = g.refx[gi] + gdx + bx0 + u0;
     const int Y0 = g.refy[gi] + gdy + by0 + v0;
     const int needw = bw + (u1 - u0), needh = bh + (v1 - v0);
@@ -203,40 +212,56 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_search_tiled(SearchLaunch 
     }
     // (e) stage the patch: rows [0, needh) x columns [0, needw); the rest
     // (reached only by zero weights or by candidates outside the zone) is zero
-    const int ph = mh + kTileV + 2 * kTT;
-    for (int e = tid; e < PITCH * ph; e += kTiledThreads) {
-      const int yy = e / PITCH, xx = e - yy * PITCH;
-      uint16_t v = 0;
-      if (yy < needh && xx < needw) v = p.cur.pix[(size_t)(Y0 + yy) * p.cur.pitch + (X0 + xx)];
-      s_patch[e] = v;
-    }
-    __syncthreads();
-    // (d) per column: extent of non-zero rows and runs of constant multiplicity
-    for (int x = tid; x < bw; x += kTiledThreads) {
-      const double* col = s_map + x * mh;
-      int lo = INT_MAX, hi = -1, nr = 0, cur_m = 0, start = 0;
-      for (int y = 0; y <= bh; ++y) {
-        const int m = y < bh ? (int)(col[y] * (1.0 / kMult)) : 0;
-        if (m != 0) {
-          lo = min(lo, y);
-          hi = y;
+    const int ph = mh + kTT * nvg + 2 * kTT;
+    constexpr int kW = kTiledThreads / 32;
+    for (int yy = warp; yy < ph; yy += 4 * kW)  // four rows' loads in flight
+      for (int xx = lane; xx < needw; xx += 32) {
+        uint16_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int y = yy + k * kW;
+          v[k] = y < needh ? p.cur.pix[(size_t)(Y0 + y) * p.cur.pitch + (X0 + xx)] : (uint16_t)0;
         }
-        if (m != cur_m) {
-          if (cur_m != 0) {
-            if (nr < kRunsPerCol) s_runs[x * kRunsPerCol + nr] = start | ((y - 1) << 8) | (cur_m << 16);
-            ++nr;
-          }
-          cur_m = m;
-          start = y;
-        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (yy + k * kW < ph) s_patch[(yy + k * kW) * PITCH + xx] = v[k];
       }
-      s_ext[x] = hi < 0 ? 1 : (lo | (hi << 16));
-      s_nrun[x] = nr;
-      if (nr > kRunsPerCol) atomicOr(&s_overflow, 1);
+    __syncthreads();
+    // (d) per column, by a warp: extent of non-zero rows and runs of constant
+    // multiplicity, whose ends are the rows (up to bh, where it is 0) at which it changes
+    for (int x = warp; x < bw; x += kTiledThreads / 32) {
+      const double* col = s_map + x * mh;
+      int lo = INT_MAX, hi = -1, nr = 0, start = 0, before = 0;
+      for (int y0 = 0; y0 <= bh; y0 += 32) {
+        const int y = y0 + lane;
+        const int m = y < bh ? (int)(col[y] * (1.0 / kMult)) : 0;
+        const int up = __shfl_up_sync(0xffffffffu, m, 1);
+        const int prev = lane > 0 ? up : before;
+        before = __shfl_sync(0xffffffffu, m, 31);
+        const unsigned on = __ballot_sync(0xffffffffu, m != 0), change = __ballot_sync(0xffffffffu, m != prev && y <= bh);
+        const unsigned ends = __ballot_sync(0xffffffffu, m != prev && y <= bh && prev != 0);
+        if (on) {
+          lo = min(lo, y0 + __ffs(on) - 1);
+          hi = y0 + 31 - __clz(on);
+        }
+        const unsigned below = (1u << lane) - 1u;
+        if ((ends >> lane) & 1u) {
+          const unsigned c = change & below;
+          const int s = c ? y0 + 31 - __clz(c) : start, k = nr + __popc(ends & below);
+          if (k < kRunsPerCol) s_runs[x * kRunsPerCol + k] = s | ((y - 1) << 8) | (prev << 16);
+        }
+        nr += __popc(ends);
+        if (change) start = y0 + 31 - __clz(change);
+      }
+      if (lane == 0) {
+        s_ext[x] = hi < 0 ? 1 : (lo | (hi << 16));
+        s_nrun[x] = nr;
+        if (nr > kRunsPerCol) atomicOr(&s_overflow, 1);
+      }
     }
     __syncthreads();
 
-    // (f) candidates: x offset u0 + lane, y offsets v0 + rb + 0..7, map columns of parity `half`
+    // (f) candidates: x offset u0 + ul, y offsets v0 + rb + 0..7, map columns of class `cls`
     double acc[kTT];
     unsigned S1[kTT];
     unsigned long long S11[kTT];
@@ -247,12 +272,12 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_search_tiled(SearchLaunch 
       S11[k] = 0;
     }
     const bool overflow = s_overflow != 0;
-    for (int x = half; x < bw; x += 2) {
+    for (int x = cls; x < bw; x += ncls) {
       const int ext = s_ext[x];
       const int lo = ext & 0xffff, hi = ext >> 16;
       if (lo > hi) continue;
       // column of this thread from row lo + rb, in blocks of 8 rows
-      const uint16_t* cp = s_patch + (lo + rb) * PITCH + x + lane;
+      const uint16_t* cp = s_patch + (lo + rb) * PITCH + x + ul;
       const double* wp = s_map + x * mh + lo;
       double A[kTT], B[kTT];
 #pragma unroll
@@ -304,7 +329,7 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_search_tiled(SearchLaunch 
         }
         if (--nchunk == 0) break;
       }
-      const uint16_t* colp = s_patch + rb * PITCH + x + lane;
+      const uint16_t* colp = s_patch + rb * PITCH + x + ul;
       if (!overflow) {
         const int nr = s_nrun[x];
         for (int q = 0; q < nr; ++q) {
@@ -345,30 +370,37 @@ __global__ void __launch_bounds__(kTiledThreads, 2) k_search_tiled(SearchLaunch 
         }
       }
     }
-    // sum the two column halves (the map is no longer needed)
+    // sum the column classes (the map is no longer needed)
     __syncthreads();
-    if (half == 1) {
+    if (cls > 0) {
+      const int slot = (cls - 1) * 32 * wpc + pair;
 #pragma unroll
       for (int k = 0; k < kTT; ++k) {
-        s_pacc[k * (kTiledThreads / 2) + pidx] = acc[k];
-        s_p11[k * (kTiledThreads / 2) + pidx] = S11[k];
-        s_p1[k * (kTiledThreads / 2) + pidx] = S1[k];
+        s_pacc[k * kTiledThreads + slot] = acc[k];
+        s_p11[k * kTiledThreads + slot] = S11[k];
+        s_p1[k * kTiledThreads + slot] = S1[k];
       }
     }
     __syncthreads();
     double bn = 0.0;
     int bi = INT_MAX;
-    if (half == 0) {
+    if (cls == 0 && active) {
       const long long Pl = P, S0 = g.s0[gi];
       const double den1 = (double)(Pl * g.s00[gi] - S0 * S0);
-      const int u = u0 + lane;
+      const int u = u0 + ul;
 #pragma unroll
       for (int k = 0; k < kTT; ++k) {
-        const double a = acc[k] + s_pacc[k * (kTiledThreads / 2) + pidx];
-        const unsigned s1k = S1[k] + s_p1[k * (kTiledThreads / 2) + pidx];
-        const unsigned long long s11k = S11[k] + s_p11[k * (kTiledThreads / 2) + pidx];
+        double a = acc[k];
+        unsigned s1k = S1[k];
+        unsigned long long s11k = S11[k];
+        for (int c = 1; c < ncls; ++c) {
+          const int slot = k * kTiledThreads + (c - 1) * 32 * wpc + pair;
+          a += s_pacc[slot];
+          s1k += s_p1[slot];
+          s11k += s_p11[slot];
+        }
         const int v = v0 + rb + k;
-        if (u > u1 || v > v1) continue;
+        if (v > v1) continue;
         const long long s01 = __double2ll_rn(a) - ((long long)s1k << kMultShift);
         const long long num = Pl * s01 - S0 * (long long)s1k;
         const long long d2 = Pl * (long long)s11k - (long long)s1k * (long long)s1k;
