@@ -81,6 +81,7 @@ struct ptk_ctx {
   // other reader at its entry (sync_cur).
   cudaStream_t copy_stream[kFrameBufs]{};
   cudaEvent_t buf_ready[kFrameBufs]{}, buf_free[kFrameBufs]{}, main_mark{nullptr};
+  SideStream side{};  // kernels beside the main stream's, between a fork and a join on it
   bool ready_pending[kFrameBufs]{};
   bool free_valid[kFrameBufs]{};
   bool released_early[kFrameBufs]{};  // the latest graph using it released it after its precompute
@@ -118,6 +119,7 @@ struct ptk_ctx {
   int* d_order{nullptr};
   int max_P{0};
   int max_R{0};
+  PowellSizes powell{};  // the same by size class
   int max_dup{1};  // largest repeat count of one offset within a pattern
   bool patterns_ok{false};
 
@@ -319,7 +321,8 @@ int upload_patterns(ptk_ctx* c) {
   const int n = c->n;
   std::vector<int> start(n + 1, 0);
   int maxP = 0;
-  double maxnorm = 0.0;
+  double maxnorm = 0.0, small_norm = 0.0;
+  int n_large = 0, small_P = 0;
   for (int i = 0; i < n; ++i) {
     const size_t P = c->h_pat[i].size();
     if (P > (size_t)kMaxPatternPoints)
@@ -327,7 +330,15 @@ int upload_patterns(ptk_ctx* c) {
     if ((long long)start[i] + (long long)P > (1ll << 30)) return fail(c, PTK_ERR_LIMIT, "too many pattern points");
     start[i + 1] = start[i] + (int)P;
     maxP = std::max(maxP, (int)P);
-    for (const short2& q : c->h_pat[i]) maxnorm = std::max(maxnorm, std::sqrt((double)q.x * q.x + (double)q.y * q.y));
+    double norm = 0.0;
+    for (const short2& q : c->h_pat[i]) norm = std::max(norm, std::sqrt((double)q.x * q.x + (double)q.y * q.y));
+    maxnorm = std::max(maxnorm, norm);
+    if ((int)P > kPowellWidePoints) {
+      ++n_large;
+    } else {
+      small_norm = std::max(small_norm, norm);
+      small_P = std::max(small_P, (int)P);
+    }
   }
   const size_t total = (size_t)start[n];
   std::vector<short2> flat;
@@ -359,6 +370,7 @@ int upload_patterns(ptk_ctx* c) {
   CK(cudaMemcpyAsync(c->d_counts, &cnt0, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   c->max_P = maxP;
   c->max_R = (int)std::ceil(maxnorm) + 1;
+  c->powell = PowellSizes{n, maxP, c->max_R, n_large, small_P, (int)std::ceil(small_norm) + 1};
   int max_dup = 1;
   for (int i = 0; i < n; ++i) {
     std::vector<int> keys;
@@ -707,12 +719,13 @@ int enqueue_subpixel(ptk_ctx* c, int method, cudaStream_t s) {
     CK(cudaMemsetAsync(lp.redo_count, 0, sizeof(int), s));
     launch_subpix_lm(c->g, frame(c, c->cur_slot), lp, s);
     if (lp.redo_list) {  // those grains: the reference's Powell from their pixel-stage state
-      launch_subpix_powell(c->g, frame(c, c->cur_slot), subpix_params(c), c->max_P, c->max_R, c->num_sms, lp.redo_list,
-                           s, lp.redo_count);
+      launch_subpix_powell(c->g, frame(c, c->cur_slot), subpix_params(c), c->powell, c->num_sms, lp.redo_list, s,
+                           c->side, lp.redo_count);
       c->launches += 1;
     }
   } else if (method == PTK_SUBPIX_POWELL) {
-    launch_subpix_powell(c->g, frame(c, c->cur_slot), subpix_params(c), c->max_P, c->max_R, c->num_sms, c->d_order, s);
+    launch_subpix_powell(c->g, frame(c, c->cur_slot), subpix_params(c), c->powell, c->num_sms, c->d_order, s, c->side);
+    if (powell_split(c->powell, c->num_sms)) c->launches += 1;
   } else {
     return fail(c, PTK_ERR_ARG, "unknown subpixel method");
   }
@@ -830,6 +843,9 @@ int ptk_create(ptk_ctx** out, const ptk_config* cfg) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->buf_free[p], cudaEventDisableTiming);
   }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->main_mark, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side.stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->side.fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->side.join, cudaEventDisableTiming);
   if (e != cudaSuccess) return bail(cuda_fail(c, e, "cudaEventCreate"));
   c->stream = c->own_stream;
   // rows of whole 16-byte units as they are (host rows and device rows then
@@ -924,6 +940,9 @@ int ptk_destroy(ptk_ctx* c) {
     if (c->buf_free[p]) cudaEventDestroy(c->buf_free[p]);
   }
   if (c->main_mark) cudaEventDestroy(c->main_mark);
+  if (c->side.stream) cudaStreamDestroy(c->side.stream);
+  if (c->side.fork) cudaEventDestroy(c->side.fork);
+  if (c->side.join) cudaEventDestroy(c->side.join);
   delete c;
   return PTK_OK;
 }
@@ -1567,7 +1586,7 @@ int ptk_track_frame(ptk_ctx* c, int num_image) {
       SearchGeom sg;
       if ((rc = search_geometry(c, l, &sg))) return rc;
     }
-    prepare_subpix(c->n, c->max_P, c->max_R, c->num_sms);
+    prepare_subpix(c->powell, c->num_sms);
     const int64_t before = c->launches;
     CK(cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeRelaxed));
     rc = enqueue_frame(c, pre, swap, c->cap_stream);
@@ -1606,7 +1625,8 @@ int ptk_track_frame(ptk_ctx* c, int num_image) {
     if ((rc = search_geometry(c, l, &sg))) return rc;
     nk += (l == 0 ? 1 : 0) + level_launches(sg);
   }
-  if (c->cfg.subpixel) nk += 1;
+  if (c->cfg.subpixel)
+    nk += c->cfg.subpix_method == PTK_SUBPIX_POWELL && powell_split(c->powell, c->num_sms) ? 2 : 1;
   c->launches += nk;
   if (swap) {
     std::swap(c->ref_slot, c->cur_slot);

@@ -187,12 +187,27 @@ void prepare_search_bf16();
 void launch_search_bf16(const Bf16Launch& p, int grid, cudaStream_t s, cudaEvent_t* ev = nullptr,
                         cudaEvent_t frame_ready = nullptr);
 void launch_end_frame(const GrainsDev& g, int swap_reference, cudaStream_t s);
-void prepare_subpix(int n, int max_points, int max_r, int num_sms);
-// order: grains by decreasing pattern size (one block each), or null for index
-// order; with list_count, only the first *list_count entries of `order` (a
-// device-built list) are refined
-void launch_subpix_powell(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, int max_points, int max_r,
-                          int num_sms, const int* order, cudaStream_t s, const int* list_count = nullptr);
+// Grains by pattern size for Powell's launches: `order` lists them by decreasing
+// size, the first n_large with more than kPowellWidePoints points; largest
+// pattern and radius of all and of the others.
+constexpr int kPowellWidePoints = 1500;
+struct PowellSizes {
+  int n, max_points, max_r;
+  int n_large, small_points, small_r;
+};
+// A stream and events for work beside the caller's stream.
+struct SideStream {
+  cudaStream_t stream;
+  cudaEvent_t fork, join;
+};
+bool powell_split(const PowellSizes& z, int num_sms);  // two launches instead of one
+void prepare_subpix(const PowellSizes& z, int num_sms);
+// order: grains by decreasing pattern size (one block each); with list_count,
+// only the first *list_count entries of `order` (a device-built list, in any
+// order) are refined
+void launch_subpix_powell(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const PowellSizes& z,
+                          int num_sms, const int* order, cudaStream_t s, const SideStream& side,
+                          const int* list_count = nullptr);
 void launch_objective(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const double* X,
                       double* f, double* grad, int max_points, cudaStream_t s);
 void launch_widen_u8(const uint8_t* src, size_t src_pitch, uint16_t* dst, int dst_pitch, int dimx, int dimy,

@@ -839,32 +839,59 @@ static bool powell_staged(int max_points) { return (size_t)max_points * 2 * size
 // grains of up to 5,000 points 18.9 -> 17.4 ms, 40 of up to 2,100 equal, 12 of
 // up to 530 1.88 -> 2.03 ms, 400 of up to 2,820 7.8 -> 8.6 ms, 2000 of up to
 // 5,000 27.2 -> 28.4 ms.
-constexpr int kPowellWidePoints = 1500;
 typedef void (*PowellKernel)(GrainsDev, FrameDev, SubpixParams, int, int, const int*, const int*);
-static PowellKernel powell_kernel(int n, int max_points, int num_sms, int* threads) {
-  if (!powell_staged(max_points)) {
-    *threads = 256;
-    return k_subpix_powell<256, 1, RefGlobal>;
+struct PowellLaunch {
+  PowellKernel kernel;
+  int threads;
+  PowellSmem smem;
+  PowellLaunch(int n, int max_points, int max_r, int num_sms, bool small) {
+    const bool staged = powell_staged(max_points), wide = n <= num_sms && max_points > kPowellWidePoints;
+    kernel = !staged ? k_subpix_powell<256, 1, RefGlobal>
+             : wide  ? k_subpix_powell<256, 2, RefStaged>
+             : small ? k_subpix_powell<128, 4, RefStaged>
+                     : k_subpix_powell<128, 3, RefStaged>;
+    threads = !staged || wide ? 256 : 128;
+    smem = powell_smem(max_points, max_r, staged);
+    ensure_smem((const void*)kernel, smem.bytes);
   }
-  const bool wide = n <= num_sms && max_points > kPowellWidePoints;
-  *threads = wide ? 256 : 128;
-  return wide ? k_subpix_powell<256, 2, RefStaged> : k_subpix_powell<128, 3, RefStaged>;
+  void operator()(int n, const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const int* order,
+                  const int* list_count, cudaStream_t s) const {
+    kernel<<<n, threads, smem.bytes, s>>>(g, cur, sp, smem.patch_cap, smem.max_points, order, list_count);
+  }
+};
+
+// One launch gives every block the shared memory of the largest pattern (5,000
+// points: two blocks an SM).  With more grains than run at once, those of up to
+// kPowellWidePoints points (29 KB: four blocks an SM) get a launch of their own,
+// beside the others', and fill the SMs that these leave idle: 2000 grains of 300
+// to 5,000 points, whole pair 26.4 -> 24.0 ms (five small blocks an SM: 23.9;
+// the large ones with 256 threads: 24.4); 400 grains of 1,260 to 2,820, which
+// all run at once, would take 6.88 instead of 6.65 ms.
+bool powell_split(const PowellSizes& z, int num_sms) {
+  return z.n > 3 * num_sms && z.n_large > 0 && z.n_large < z.n;
 }
 
-void prepare_subpix(int n, int max_points, int max_r, int num_sms) {
-  int threads;
-  const PowellKernel k = powell_kernel(n, max_points, num_sms, &threads);
-  ensure_smem((const void*)k, powell_smem(max_points, max_r, powell_staged(max_points)).bytes);
+void prepare_subpix(const PowellSizes& z, int num_sms) {
+  PowellLaunch(z.n, z.max_points, z.max_r, num_sms, false);
+  if (powell_split(z, num_sms)) PowellLaunch(z.n, z.small_points, z.small_r, num_sms, true);
 }
 
-void launch_subpix_powell(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, int max_points, int max_r,
-                          int num_sms, const int* order, cudaStream_t s, const int* list_count) {
+void launch_subpix_powell(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const PowellSizes& z,
+                          int num_sms, const int* order, cudaStream_t s, const SideStream& side,
+                          const int* list_count) {
   if (g.n <= 0) return;
-  prepare_subpix(g.n, max_points, max_r, num_sms);
-  int threads;
-  const PowellKernel k = powell_kernel(g.n, max_points, num_sms, &threads);
-  const PowellSmem m = powell_smem(max_points, max_r, powell_staged(max_points));
-  k<<<g.n, threads, m.bytes, s>>>(g, cur, sp, m.patch_cap, max_points, order, list_count);
+  const PowellLaunch large(z.n, z.max_points, z.max_r, num_sms, false);
+  if (list_count || !powell_split(z, num_sms)) {
+    large(g.n, g, cur, sp, order, list_count, s);
+    return;
+  }
+  const PowellLaunch small(z.n, z.small_points, z.small_r, num_sms, true);
+  cudaEventRecord(side.fork, s);
+  cudaStreamWaitEvent(side.stream, side.fork, 0);
+  large(z.n_large, g, cur, sp, order, nullptr, s);
+  small(z.n - z.n_large, g, cur, sp, order + z.n_large, nullptr, side.stream);
+  cudaEventRecord(side.join, side.stream);
+  cudaStreamWaitEvent(s, side.join, 0);
 }
 
 void launch_objective(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const double* X, double* f,

@@ -60,14 +60,15 @@ def test_objective_is_the_serial_loop(ptk, oracle, cuda_device, kind):
     t.close()
 
 
-@pytest.mark.parametrize("n,interp", [(40, "cubic"), (200, "cubic"), (40, "linear"), (40, "quintic")])
+@pytest.mark.parametrize("n,interp", [(40, "cubic"), (200, "cubic"), (470, "cubic"), (40, "linear"), (40, "quintic")])
 def test_refinement_takes_the_reference_path(ptk, wl, oracle, cuda_device, n, interp):
-    """Powell's result bit for bit (both kernel widths: fewer grains than SMs
-    and more), on the grains whose angles the C library rounds correctly: about
+    """Powell's result bit for bit (fewer grains than SMs, more, and more than run
+    at once, in two size classes), on the grains whose angles the C library rounds correctly: about
     one sine in 420 is not, and a grain visits some 100 angles, so that about
     0.79 of the grains are expected to be equal; the others stay within 1e-5 px."""
-    p = dict(wl.PRESETS["small16"], dimx=1536, dimy=1024, n=n, mix=[(0.5, 8.0, 18.0), (0.5, 22.0, 30.0)])
+    p = dict(wl.PRESETS["small16"], dimx=1536, dimy=1024 if n < 300 else 2400, n=n, mix=[(0.5, 8.0, 18.0), (0.5, 22.0, 30.0)])
     pair = wl.make_pair(p, seed=5)
+    assert len(pair["rec"]) == n
     o = wl.tracker_options(p)
     t = ptk.Tracker(p["dimx"], p["dimy"], image_interpolator=interp, iraz=100, **o)
     t.set_grains(pair["rec"])
