@@ -80,9 +80,10 @@ __device__ __forceinline__ SeqPlan seq_plan(int P, int G) {
 }
 
 // Threads of a block that form one of NS sums side by side: all of its share, up
-// to 128 (more threads shorten the chunks less than they lengthen the scan).
+// to 128, or 256 in the widest blocks, which have the largest patterns (more
+// threads shorten the chunks less than they lengthen the scan).
 template <int NT, int NS>
-constexpr int kSeqThreads = NT / NS < 128 ? NT / NS : 128;
+constexpr int kSeqThreads = NT >= 512 ? 256 : (NT / NS < 128 ? NT / NS : 128);
 
 // NS = 1 or 2 sums of P terms, each by kSeqThreads<NT, NS> threads (plan:
 // seq_plan(P, kSeqThreads<NT, NS>)).  terms.of(n) provides sum n's terms as a

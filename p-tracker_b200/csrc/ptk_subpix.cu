@@ -699,7 +699,7 @@ __host__ __device__ inline size_t powell_vals_offset(int patch_cap) {
 constexpr size_t kTermPad = 4 * sizeof(double);
 
 // what a block may use besides the kernels' static shared memory
-constexpr size_t kPowellSmemMax = (227 - 12) * 1024;
+constexpr size_t kPowellSmemMax = (227 - 20) * 1024;
 
 // Margin of the staged frame region around the pattern (pixels): the moves of
 // Powell's steps.  Samples further out read the frame.
@@ -834,23 +834,26 @@ static PowellSmem powell_smem(int max_points, int max_r, bool staged) {
 static bool powell_staged(int max_points) { return (size_t)max_points * 2 * sizeof(double) <= kPowellSmemMax - 32 * 1024; }
 
 // The kernel of a launch.  128 threads a block, except where there are no more
-// grains than SMs (each block has an SM to itself, and its evaluations'
-// latency is the whole time) and patterns large enough to keep 256 busy: 80
-// grains of up to 5,000 points 18.9 -> 17.4 ms, 40 of up to 2,100 equal, 12 of
-// up to 530 1.88 -> 2.03 ms, 400 of up to 2,820 7.8 -> 8.6 ms, 2000 of up to
-// 5,000 27.2 -> 28.4 ms.
+// grains than SMs (each block has an SM to itself, and its evaluations' latency
+// is the whole time) and patterns large enough to keep 256 or 512 busy.  Threads
+// a block 128 / 256 / 512: 80 grains of up to 5,000 points (three frames with
+// rescues) 18.9 / 18.2 / 16.4 ms, 40 of up to 2,100 2.72 / 2.70 / 2.76 ms, 12 of
+// up to 530 1.88 / 2.03 / 2.6 ms; 400 of up to 2,820 7.8 / 8.6 / 11.1 ms, 2000 of
+// up to 5,000 27.2 / 28.4 / 41 ms.
+constexpr int kPowellWidestPoints = 3000;
 typedef void (*PowellKernel)(GrainsDev, FrameDev, SubpixParams, int, int, const int*, const int*);
 struct PowellLaunch {
   PowellKernel kernel;
   int threads;
   PowellSmem smem;
   PowellLaunch(int n, int max_points, int max_r, int num_sms, bool small) {
-    const bool staged = powell_staged(max_points), wide = n <= num_sms && max_points > kPowellWidePoints;
-    kernel = !staged ? k_subpix_powell<256, 1, RefGlobal>
-             : wide  ? k_subpix_powell<256, 2, RefStaged>
-             : small ? k_subpix_powell<128, 4, RefStaged>
-                     : k_subpix_powell<128, 3, RefStaged>;
-    threads = !staged || wide ? 256 : 128;
+    const bool staged = powell_staged(max_points);
+    threads = !staged ? 256 : (n > num_sms || max_points <= kPowellWidePoints ? 128 : (max_points <= kPowellWidestPoints ? 256 : 512));
+    kernel = !staged         ? k_subpix_powell<256, 1, RefGlobal>
+             : threads == 512 ? k_subpix_powell<512, 1, RefStaged>
+             : threads == 256 ? k_subpix_powell<256, 2, RefStaged>
+             : small          ? k_subpix_powell<128, 4, RefStaged>
+                              : k_subpix_powell<128, 3, RefStaged>;
     smem = powell_smem(max_points, max_r, staged);
     ensure_smem((const void*)kernel, smem.bytes);
   }
