@@ -39,6 +39,17 @@ __device__ __forceinline__ double cubic_px_twice(int p0, int p1, int p2, int p3,
   return __fma_rn(2.0, (double)p1, a * x2 * x + b * x2 + c * x);
 }
 
+// cubic_px_twice, and twice the derivative with respect to x:
+// 3 a x x + 2 b x + c in that order.
+__device__ __forceinline__ double cubic_px_twice(int p0, int p1, int p2, int p3, double x, double x2, double* dx) {
+  const int d = p1 - p2, t = p3 - p0;
+  const double a = (double)(3 * d + t);
+  const double b = (double)(p0 - p1 - t - 4 * d);
+  const double c = (double)(p2 - p0);
+  *dx = 3.0 * a * x * x + 2.0 * b * x + c;
+  return __fma_rn(2.0, (double)p1, a * x2 * x + b * x2 + c * x);
+}
+
 // cubic1 with its multiplications by 2 and 1/2 folded: they are exact, so a
 // fused multiply-add by them rounds once, where the addition does.
 __device__ __forceinline__ double cubic1_fast(double p0, double p1, double p2, double p3, double x) {

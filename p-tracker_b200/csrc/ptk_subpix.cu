@@ -90,10 +90,26 @@ __device__ __forceinline__ double quintic1(double p0, double p1, double p2, doub
   return (a * x4 * x + b * x4 + c * x2 * x + d * x2 + e * x + f);
 }
 
+// Whether the cubic's 4x4 support of (x, y) lies in the frame.
+__device__ __forceinline__ bool cubic_inside(const FrameDev& f, double x, double y) {
+  return x >= 1.0 && y >= 1.0 && x < (double)(f.dimx - 2) && y < (double)(f.dimy - 2);
+}
+
 // image_interp*::getValue (src/interpol.cpp:21-39, 55-86, 113-144).  The
 // reference reads out of bounds when the support leaves the frame; here the
 // support is clamped into the frame and *clamped is set.
 __device__ double interp(const FrameDev& f, int kind, double x, double y, bool* clamped) {
+  if (kind == PTK_INTERP_CUBIC && cubic_inside(f, x, y)) {
+    int ix, iy;
+    const double x01 = split(x, &ix), y01 = split(y, &iy), y2 = y01 * y01;
+    const uint16_t* p = f.pix + (size_t)(iy - 1) * f.pitch + (ix - 1);
+    double arr[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      arr[i] = cubic_px_twice(__ldg(p + i), __ldg(p + f.pitch + i), __ldg(p + 2 * f.pitch + i), __ldg(p + 3 * f.pitch + i),
+                              y01, y2);
+    return 0.5 * cubic1_fast(arr[0], arr[1], arr[2], arr[3], x01);
+  }
   int ix = (int)floor(x);
   int iy = (int)floor(y);
   const double x01 = x - (double)ix;
@@ -125,6 +141,20 @@ __device__ double interp(const FrameDev& f, int kind, double x, double y, bool* 
 
 // Cubic value and its partial derivatives at (x, y).
 __device__ double interp_cubic_grad(const FrameDev& f, double x, double y, double* gx, double* gy, bool* clamped) {
+  if (cubic_inside(f, x, y)) {  // everything below on doubled values
+    int ix, iy;
+    const double x01 = split(x, &ix), y01 = split(y, &iy), y2 = y01 * y01;
+    const uint16_t* p = f.pix + (size_t)(iy - 1) * f.pitch + (ix - 1);
+    double arr[4], darr[4], w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      arr[i] = cubic_px_twice(__ldg(p + i), __ldg(p + f.pitch + i), __ldg(p + 2 * f.pitch + i), __ldg(p + 3 * f.pitch + i),
+                              y01, y2, &darr[i]);
+    cubic_weights(x01, w);
+    *gx = 0.5 * cubic1_dx(arr[0], arr[1], arr[2], arr[3], x01);
+    *gy = 0.5 * (w[0] * darr[0] + w[1] * darr[1] + w[2] * darr[2] + w[3] * darr[3]);
+    return 0.5 * cubic1_fast(arr[0], arr[1], arr[2], arr[3], x01);
+  }
   int ix = (int)floor(x);
   int iy = (int)floor(y);
   const double x01 = x - (double)ix;
