@@ -1664,12 +1664,13 @@ static int objective_common(ptk_ctx* c, const double* X3n, double* f, double* g3
     CK(cudaMalloc(&c->d_gr, sizeof(double) * 3 * n));
   }
   CK(cudaMemcpyAsync(c->d_X, X3n, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
-  if (g3n && c->cfg.subpix_method == PTK_SUBPIX_ADJOINT_LM)
+  if (g3n && c->cfg.subpix_method == PTK_SUBPIX_ADJOINT_LM) {
     launch_grad_f32(c->g, frame(c, c->cur_slot), c->d_X, c->d_f, c->d_gr, c->stream);  // the LM's FP32 adjoint
-  else
-    launch_objective(c->g, frame(c, c->cur_slot), subpix_params(c), c->d_X, c->d_f, g3n ? c->d_gr : nullptr,
-                     c->max_P, c->stream);
-  c->launches += 1;
+    c->launches += 1;
+  } else {
+    c->launches += launch_objective(c->g, frame(c, c->cur_slot), subpix_params(c), c->d_X, c->d_f,
+                                    g3n ? c->d_gr : nullptr, c->powell, c->num_sms, c->d_order, c->stream, c->side);
+  }
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(f, c->d_f, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
   if (g3n) CK(cudaMemcpyAsync(g3n, c->d_gr, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->stream));

@@ -208,8 +208,10 @@ void prepare_subpix(const PowellSizes& z, int num_sms);
 void launch_subpix_powell(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const PowellSizes& z,
                           int num_sms, const int* order, cudaStream_t s, const SideStream& side,
                           const int* list_count = nullptr);
-void launch_objective(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const double* X,
-                      double* f, double* grad, int max_points, cudaStream_t s);
+// returns the number of launches
+int launch_objective(const GrainsDev& g, const FrameDev& cur, const SubpixParams& sp, const double* X, double* f,
+                     double* grad, const PowellSizes& z, int num_sms, const int* order, cudaStream_t s,
+                     const SideStream& side);
 void launch_widen_u8(const uint8_t* src, size_t src_pitch, uint16_t* dst, int dst_pitch, int dimx, int dimy,
                      cudaStream_t s);
 void launch_remap_build(const double* params14, const double* trig4, double2* map, int dimx, int dimy,
