@@ -111,6 +111,7 @@ constexpr int kStageBoxRows = 8;  // image rows per TMA box of the strip staging
 constexpr long kDrainLimit = 1L << 26;
 // operand rows in flight: W_r and M_r of one footprint row per ring buffer
 constexpr int kRowThread = 32;  // issues the operand rows' copies during the MMA phases
+constexpr int kNextWarp = 2;    // fetches the next work item during a tile's first MMA phase
 constexpr int kRing = 8;       // barrier slots
 constexpr int kRingUsed = 4;   // buffers
 // weights kernel: 512 threads, 108 KB of 32-bit maps (two blocks per SM, as
@@ -155,6 +156,16 @@ __host__ __device__ inline Geom geom_of(int half, int nb = kRingUsed, int nx = 4
   g.nb = nb;
   return g;
 }
+
+// A work item of the search kernel: (list entry, tile) and what it needs of the
+// grain.
+struct SearchItem {
+  int item, gi, b, P;
+  int skip;         // not searched: masked, outside the frame, no pattern
+  int half;
+  int X, Y;         // integer position: refcoord + round(d)
+  float mean0, c00_rsqrt;
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -447,14 +458,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
   // kRowThread, with a barrier between their turns) and consumed (thread 0) so far (a buffer's barriers complete one phase per use)
   __shared__ unsigned s_iss[kRing], s_con[kRing];
   __shared__ uint32_t s_tmem;
-  __shared__ int s_li, s_err, s_bb[4];
-  __shared__ double2 s_cs[kNRot];
-  __shared__ float2 s_csf[kNRot];
+  __shared__ int s_err, s_bb[4];
+  __shared__ SearchItem s_next;                          // the next item, once s_next_ready
+  __shared__ int s_next_ready;
+  __shared__ double2 s_cs[kNRot], s_next_cs[kNRot];      // cos / sin of the rotation steps
   __shared__ float s_cv[kWarps * kBf16KeepMax];
   __shared__ int s_ci[kWarps * kBf16KeepMax];
   __shared__ int s_kept[kBf16KeepMax], s_nkept;  // the tile's kept candidates (packed u, v) and their count
-  __shared__ float s_rel;
-  __shared__ unsigned char s_rng[2 * kMaxFoot];
+  __shared__ float s_rel, s_wtop[kWarps];
+  __shared__ unsigned char s_rng[2 * kMaxFoot], s_next_rng[2 * kMaxFoot];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t mbar = smem_u32(&s_mbar);
 
@@ -472,6 +484,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_probe)));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_stage)));
     s_stage_out = 0;
+    s_next_ready = 0;
     asm volatile("fence.mbarrier_init.release.cluster;");
     s_err = 0;
     for (int k = 0; k < kRing; ++k) s_iss[k] = s_con[k] = 0u;
@@ -497,8 +510,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
     }
   }
   int zhalf = -1;  // footprint geometry whose zero blocks the operand rows hold
-  int pf_next = -1;   // thread 0: the next work item, taken before this one's epilogue (-1: none)
-  bool pf = false;    // thread 0: its first operand rows and image strip are already on their way
+  bool pf = false;    // thread 0: this item's first operand rows and image strip are already on their way
 
   const GrainsDev& g = p.g;
   const int count = *p.list_count;
@@ -506,48 +518,71 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
   const int keep = p.keep;
   const uint32_t idesc = idesc_of(p.ny);
 
+  // Takes the next work item (warp kNextWarp): four dependent memory accesses,
+  // which the tile in progress hides.
+  auto fetch_next = [&]() {
+    int item = 0;
+    if (lane == 0) item = atomicAdd(p.work_next, 1);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    const int li = item / tiles;
+    if (li < count) {
+      const int gi = p.list[li];
+      const int b = g.pstart[gi], P = g.pstart[gi + 1] - b, half = p.half[gi];
+      const bool skip = g.masked[gi] || (g.flags[gi] & 2) || P <= 0 || P > kMaxPatternPoints;
+      if (lane == 0) {
+        const double c0c0 = g.c0c0[gi];
+        s_next = SearchItem{item, gi, b, P, skip ? 1 : 0, half, g.refx[gi] + (int)round(g.dx[gi]),
+                            g.refy[gi] + (int)round(g.dy[gi]), (float)g.mean0[gi],
+                            c0c0 > 0.0 ? (float)(1.0 / sqrt(c0c0)) : 0.0f};
+      }
+      if (!skip) {
+        if (lane < p.nrot) s_next_cs[lane] = p.rot_cs[(size_t)gi * kNRot + lane];  // the weights kernel's, of this grain's steps
+        // the footprint rows' occupied blocks, over the blocks that share the
+        // rotation steps: the first block's minimum, the last one's maximum
+        const Geom G = geom_of(half, RING, p.nx, p.ny);
+        const unsigned char* rng = reinterpret_cast<const unsigned char*>(
+            reinterpret_cast<const uint4*>(p.wslots) + p.wofs[gi] + 2 * (size_t)G.fw * G.nbf * p.nrot);
+        for (int e = lane; e < 2 * G.fw; e += 32) {
+          int v = rng[e];
+          for (int k = 1; k < p.wsplit; ++k) v = e & 1 ? max(v, (int)rng[e + 2 * G.fw * k]) : min(v, (int)rng[e + 2 * G.fw * k]);
+          s_next_rng[e] = (unsigned char)v;
+        }
+      }
+    } else if (lane == 0) {
+      s_next.item = item;
+    }
+    if (lane == 0) s_next_ready = 1;
+  };
+
   for (;;) {
     __syncthreads();  // every thread is done with the previous grain's shared state
+    if (!s_next_ready) {
+      __syncthreads();
+      if (warp == kNextWarp) fetch_next();
+      __syncthreads();
+    }
+    // work item = (list entry, tile): the tiles of a large zone (rescues)
+    // spread over CTAs instead of running one after another in one
+    const SearchItem it = s_next;
+    const int item = it.item, li = item / tiles, t_item = item - li * tiles;
+    if (li >= count || s_err) break;
+    if (tid < kNRot) s_cs[tid] = s_next_cs[tid];
+    if (tid < 2 * kMaxFoot) s_rng[tid] = s_next_rng[tid];
+    __syncthreads();
     if (tid == 0) {
-      s_li = pf_next >= 0 ? pf_next : atomicAdd(p.work_next, 1);
-      pf_next = -1;
+      s_next_ready = 0;
       s_bb[0] = s_bb[2] = INT_MAX;
       s_bb[1] = s_bb[3] = INT_MIN;
     }
-    __syncthreads();
-    // work item = (list entry, tile): the tiles of a large zone (rescues)
-    // spread over CTAs instead of running one after another in one
-    const int item = s_li;
-    const int li = item / tiles, t_item = item - li * tiles;
-    if (li >= count || s_err) break;
-    const int gi = p.list[li];
-    const int b = g.pstart[gi], P = g.pstart[gi + 1] - b;
+    const int gi = it.gi, b = it.b, P = it.P;
     int2* topk_g = p.topk + (size_t)li * tiles * kBf16KeepMax;
-    if (g.masked[gi] || (g.flags[gi] & 2) || P <= 0 || P > kMaxPatternPoints) {
+    if (it.skip) {
       if (tid < kBf16KeepMax) topk_g[(size_t)t_item * kBf16KeepMax + tid] = make_int2(INT_MIN, INT_MIN);
       if (tid == 0) p.tile_top[item] = -INFINITY;
       continue;
     }
-    // rotation cos/sin (total_rot = base_rot + step, as the exact search) and
-    // the grain's footprint geometry
-    if (tid < p.nrot) {  // the weights kernel's cos / sin of this grain's steps
-      const double2 cs = p.rot_cs[(size_t)gi * kNRot + tid];
-      s_cs[tid] = cs;
-      s_csf[tid] = make_float2((float)cs.x, (float)cs.y);
-    }
-    const Geom G = geom_of(p.half[gi], RING, p.nx, p.ny);
-    const float mean0 = (float)g.mean0[gi];
-    const float c00_rsqrt = g.c0c0[gi] > 0.0 ? (float)(1.0 / sqrt(g.c0c0[gi])) : 0.0f;
-    const int gdx = (int)round(g.dx[gi]), gdy = (int)round(g.dy[gi]);
-    const size_t wrows = (size_t)G.fw * G.nbf * p.nrot;
-    const uint4* slotW = reinterpret_cast<const uint4*>(p.wslots) + p.wofs[gi];
-    const uint4* slotM = slotW + wrows;
-    if (tid < 2 * G.fw) {  // over the blocks that share the rotation steps: the first block's minimum, the last one's maximum
-      const unsigned char* rng = reinterpret_cast<const unsigned char*>(slotM + wrows) + tid;
-      int v = rng[0];
-      for (int k = 1; k < p.wsplit; ++k) v = tid & 1 ? max(v, (int)rng[2 * G.fw * k]) : min(v, (int)rng[2 * G.fw * k]);
-      s_rng[tid] = (unsigned char)v;
-    }
+    const Geom G = geom_of(it.half, RING, p.nx, p.ny);
+    const float mean0 = it.mean0, c00_rsqrt = it.c00_rsqrt;
     const CUtensorMap* tmap = p.tmaps + gi;  // this grain's operand rows, rotation slots zero-filled to 32
     const CUtensorMap* fmap = p.frame_tmaps + (G.hb >> 1);  // the frame's map for this Hankel width
     if (tid == 0 || tid == kRowThread)
@@ -587,7 +622,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
       const int v0 = -p.up + tv * kTileV, v1 = min(v0 + kTileV - 1, p.down);
       int2* topk = topk_g + (size_t)t * kBf16KeepMax;
       {  // the union of the rotated footprints over the tile's candidates must stay in the frame
-        const int X = g.refx[gi] + gdx, Y = g.refy[gi] + gdy;
+        const int X = it.X, Y = it.Y;
         bool oob = X + bbx0 + u0 < 0 || Y + bby0 + v0 < 0 || X + bbx1 + u1 >= p.cur.dimx ||
                    Y + bby1 + v1 >= p.cur.dimy;
         if (oob && !exact_bb) {
@@ -595,7 +630,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
           for (int i = tid; i < P; i += kThreads) {
             const short2 q0 = g.pat[b + i];
             for (int r = 0; r < p.nrot; ++r) {
-              const short2 q = rotate_round_fast(q0, s_csf[r].x, s_csf[r].y, s_cs[r].x, s_cs[r].y);
+              const short2 q = rotate_round_fast(q0, (float)s_cs[r].x, (float)s_cs[r].y, s_cs[r].x, s_cs[r].y);
               xmn = min(xmn, (int)q.x);
               xmx = max(xmx, (int)q.x);
               ymn = min(ymn, (int)q.y);
@@ -632,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
         }
       }
       // image origin of footprint column 0 at candidate (u0, v0)
-      const int Xi = g.refx[gi] + gdx - G.half + u0, Yi = g.refy[gi] + gdy - G.half + v0;
+      const int Xi = it.X - G.half + u0, Yi = it.Y - G.half + v0;
       // A strip's image rows (columns Xa .. Xa + 8 hb + 15, rows from Yi + ys)
       // are staged in shared memory by TMA boxes of 8 rows from the frame's
       // tensor map for this Hankel width, issued by thread 0 - for the next
@@ -765,6 +800,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
           mma_commit(mbar);
           committed = true;
         }
+        if (warp == kNextWarp && ys == 0) fetch_next();
         if (tid == kRowThread && !s_err) {
           for (int y = ys + NB - 1; y < min(ys + nr + NB - 1, G.fw); ++y)
             if (!issue_row(y)) {
@@ -788,37 +824,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
       }
       if (s_err) break;
 
-      // Prefetch (thread 0): the next work item is taken now and, when its
-      // grain has this footprint geometry (same shared-memory layout, zero
-      // blocks in place) and its tile lies in the frame by the +-(half - 1)
-      // bound (so that it is searched, not skipped), its first operand rows
-      // and its first strip's image rows are issued into the ring and the
-      // staging rows, which this tile no longer reads, to land during this
-      // tile's epilogue.
+      // Prefetch (thread 0): when the next work item's grain has this footprint
+      // geometry (same shared-memory layout, zero blocks in place) and its tile
+      // lies in the frame by the +-(half - 1) bound (so that it is searched, not
+      // skipped), its first operand rows and its first strip's image rows are
+      // issued into the ring and the staging rows, which this tile no longer
+      // reads, to land during this tile's epilogue.
       if (tid == 0) {
-        pf_next = atomicAdd(p.work_next, 1);
-        const int li2 = pf_next / tiles, t2 = pf_next - li2 * tiles;
-        if (li2 < count) {
-          const int gi2 = p.list[li2];
-          const int P2 = g.pstart[gi2 + 1] - g.pstart[gi2];
-          if (!(g.masked[gi2] || (g.flags[gi2] & 2) || P2 <= 0 || P2 > kMaxPatternPoints) && p.half[gi2] == G.half) {
-            const int tu2 = t2 / p.tiles_v, tv2 = t2 - tu2 * p.tiles_v;
-            const int u0b = -p.left + tu2 * kTileU, u1b = min(u0b + kTileU - 1, p.right);
-            const int v0b = -p.up + tv2 * kTileV, v1b = min(v0b + kTileV - 1, p.down);
-            const int X2 = g.refx[gi2] + (int)round(g.dx[gi2]), Y2 = g.refy[gi2] + (int)round(g.dy[gi2]);
-            const int e = G.half - 1;
-            if (X2 - e + u0b >= 0 && Y2 - e + v0b >= 0 && X2 + e + u1b < p.cur.dimx && Y2 + e + v1b < p.cur.dimy) {
-              const CUtensorMap* tm2 = p.tmaps + gi2;
-              asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tm2) : "memory");
-              pf = true;
-              for (int y = 0; y < min(NB - 1, G.fw); ++y)
-                if (!issue_row_of(tm2, y)) {
-                  s_err = 1;
-                  atomicOr(p.error, 1);
-                  break;
-                }
-              if (!s_err) stage_rows_at((X2 - G.half + u0b) & ~7, Y2 - G.half + v0b, 0);
-            }
+        const int li2 = s_next.item / tiles, t2 = s_next.item - li2 * tiles;
+        if (li2 < count && !s_next.skip && s_next.half == G.half) {
+          const int tu2 = t2 / p.tiles_v, tv2 = t2 - tu2 * p.tiles_v;
+          const int u0b = -p.left + tu2 * kTileU, u1b = min(u0b + kTileU - 1, p.right);
+          const int v0b = -p.up + tv2 * kTileV, v1b = min(v0b + kTileV - 1, p.down);
+          const int X2 = s_next.X, Y2 = s_next.Y, e = G.half - 1;
+          if (X2 - e + u0b >= 0 && Y2 - e + v0b >= 0 && X2 + e + u1b < p.cur.dimx && Y2 + e + v1b < p.cur.dimy) {
+            const CUtensorMap* tm2 = p.tmaps + s_next.gi;
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tm2) : "memory");
+            pf = true;
+            for (int y = 0; y < min(NB - 1, G.fw); ++y)
+              if (!issue_row_of(tm2, y)) {
+                s_err = 1;
+                atomicOr(p.error, 1);
+                break;
+              }
+            if (!s_err) stage_rows_at((X2 - G.half + u0b) & ~7, Y2 - G.half + v0b, 0);
           }
         }
       }
@@ -846,8 +875,52 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
         const int ul = 24 - 8 * q + (lane & 7), vl = 8 * h + 4 * ch + (lane >> 3);
         sc[ch] = (u0 + ul <= u1 && v0 + vl <= v1 && mine != INT_MIN) ? key2f(mine) : -INFINITY;
       }
-      // per-warp best `keep` (down to kKeepRelWeak below the warp's best: the
-      // tile's best is at least as high), then the block's best `keep` among them
+      // The tile's best score, and the candidates within `rel` of it: where they
+      // are no more than `keep`, they are the kept ones, in any order (a sharp
+      // texture's usual case).  With the next item fetched during the MMAs
+      // instead of after the tile (four dependent accesses), zone +-16, 4,000
+      // grains: 618 -> 594 us; +-8, 400 grains (more near candidates than are
+      // kept, one tile a CTA or two): 141 -> 143 us.  Ranking the near candidates
+      // by counting instead of the two rounds below was no faster (600, 144).
+      {
+        const int m = __reduce_max_sync(0xffffffffu, f2key(fmaxf(sc[0], sc[1])));
+        if (lane == 0) s_wtop[warp] = key2f(m);
+        if (tid == 0) s_nkept = 0;
+      }
+      __syncthreads();
+      const float tile_best = key2f(__reduce_max_sync(0xffffffffu, f2key(s_wtop[lane & (kWarps - 1)])));
+      // D / sqrt(S) <= NCC sqrt(C0C0)
+      const float keep_rel = tile_best * c00_rsqrt >= kGoodMatch ? kKeepRel : kKeepRelWeak;
+      if (tile_best > 0.0f) {
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+          const unsigned near = __ballot_sync(0xffffffffu, sc[ch] >= tile_best * (1.0f - keep_rel));
+          if (!near) continue;
+          int at = 0;
+          if (lane == 0) at = atomicAdd(&s_nkept, __popc(near));
+          at = __shfl_sync(0xffffffffu, at, 0) + __popc(near & ((1u << lane) - 1u));
+          if (((near >> lane) & 1u) && at < keep) {
+            const int ul = 24 - 8 * q + (lane & 7), vl = 8 * h + 4 * ch + (lane >> 3);
+            s_kept[at] = (ul << 8) | vl;
+          }
+        }
+      }
+      __syncthreads();
+      const int n_near = s_nkept;
+      const bool few = tile_best > 0.0f && n_near <= keep;  // (block-uniform)
+      if (few) {
+        if (tid < kBf16KeepMax) {
+          const int pk = tid < n_near ? s_kept[tid] : 0;
+          topk[tid] = tid < n_near ? make_int2(u0 + (pk >> 8), v0 + (pk & 0xff)) : make_int2(INT_MIN, INT_MIN);
+        }
+        if (tid == 0) {
+          p.tile_top[(size_t)li * tiles + t] = tile_best;
+          s_rel = keep_rel;
+        }
+      } else {
+      // More of them: the best `keep`.  Per-warp best `keep` (down to kKeepRelWeak
+      // below the warp's best: the tile's best is at least as high), then the
+      // block's best `keep` among them
       float wtop = -INFINITY;
       for (int k = 0; k < keep; ++k) {
         const int bc = sc[1] > sc[0] ? 1 : (sc[0] > -INFINITY ? 0 : -1);
@@ -941,6 +1014,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
             }
           }
         }
+      }
       }
       __syncthreads();
       // rotation steps to rescore at each kept candidate: those whose score lies
