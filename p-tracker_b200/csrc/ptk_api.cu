@@ -158,7 +158,8 @@ struct ptk_ctx {
   double2* d_map{nullptr};
   bool map_valid{false};
 
-  // objective buffers
+  // objective buffers, for obj_cap grains
+  size_t obj_cap{0};
   double* d_X{nullptr};
   double* d_f{nullptr};
   double* d_gr{nullptr};
@@ -1658,10 +1659,16 @@ static int objective_common(ptk_ctx* c, const double* X3n, double* f, double* g3
   if (g3n && (size_t)c->max_P * 24 > 227 * 1024) return fail(c, PTK_ERR_LIMIT, "pattern too large for ptk_grad");
   if (c->need_precompute && (rc = ptk_precompute(c))) return rc;
   const size_t n = (size_t)c->n;
-  if (!c->d_X) {
+  if (n > c->obj_cap) {
+    cudaFree(c->d_X);  // (the calls that used them have returned, results read back)
+    cudaFree(c->d_f);
+    cudaFree(c->d_gr);
+    c->d_X = c->d_f = c->d_gr = nullptr;
+    c->obj_cap = 0;
     CK(cudaMalloc(&c->d_X, sizeof(double) * 3 * n));
     CK(cudaMalloc(&c->d_f, sizeof(double) * n));
     CK(cudaMalloc(&c->d_gr, sizeof(double) * 3 * n));
+    c->obj_cap = n;
   }
   CK(cudaMemcpyAsync(c->d_X, X3n, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
   if (g3n && c->cfg.subpix_method == PTK_SUBPIX_ADJOINT_LM) {

@@ -85,3 +85,29 @@ def test_refinement_takes_the_reference_path(ptk, wl, oracle, cuda_device, n, in
     assert same.mean() >= 0.5, same.mean()
     assert np.abs(got[:, 4:6] - want[:, 4:6]).max() <= 1e-5
     t.close()
+
+
+def test_objective_after_more_grains(ptk, cuda_device):
+    """The objective's and gradient's buffers follow the grain count: a tracker
+    that is given many more grains answers as a new one does."""
+    rng = np.random.default_rng(0)
+    ref = rng.integers(0, 65536, (240, 240)).astype(np.uint16)
+    cur = np.roll(ref, 1, 0)
+    xy = np.stack(np.meshgrid(np.arange(-5, 6), np.arange(-5, 6)), -1).reshape(-1, 2)
+
+    def answers(counts):
+        t = ptk.Tracker(240, 240)
+        for n in counts:
+            rec = np.zeros((n, 13))
+            rec[:, 0], rec[:, 1] = 40 + np.arange(n) % 160, 40 + np.arange(n) // 160
+            t.set_grains(rec)
+            t.set_patterns([xy] * n)
+            t.load_frame(0, ref)
+            t.load_frame(1, cur)
+            t.precompute()
+            out = t.objective(np.full((n, 3), 0.25)), *t.grad(np.full((n, 3), 0.25))
+        t.close()
+        return out
+
+    for a, b in zip(answers((4, 20000)), answers((20000,))):
+        np.testing.assert_array_equal(a, b)
