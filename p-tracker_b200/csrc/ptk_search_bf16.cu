@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_search_bf16(Bf16Launch p) {
       // The tile's best score, and the candidates within `rel` of it: where they
       // are no more than `keep`, they are the kept ones, in any order (a sharp
       // texture's usual case).  With the next item fetched during the MMAs
-      // instead of after the tile (four dependent accesses), zone +-16, 4,000
+      // instead of after the tile (four dependent accesses), zone +-15, 2000
       // grains: 618 -> 594 us; +-8, 400 grains (more near candidates than are
       // kept, one tile a CTA or two): 141 -> 143 us.  Ranking the near candidates
       // by counting instead of the two rounds below was no faster (600, 144).

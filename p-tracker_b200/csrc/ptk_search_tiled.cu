@@ -85,6 +85,8 @@ __host__ __device__ inline TiledGeom tiled_geom(int max_r) {
   t.mw = box;
   // a column's last chunk ends up to 7 rows below its last point; the last
   // thread's blocks of 8 rows go 24 + 16 rows further
+  // (16 rows less in both than a chunk more each, so that offsets to +-61 fit
+  // where +-59 did: at 60, 60 grains, 2.39 ms in the direct kernel, 0.51 here)
   t.mh = ((box + kTT - 1) / kTT) * kTT + kTT;
   t.ph = t.mh + kTileV + kTT;
   return t;

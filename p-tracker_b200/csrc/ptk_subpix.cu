@@ -743,7 +743,7 @@ constexpr int kPatchMargin = 6;
 // divisions and roots), against 33k with the sums and the cosine's series in one
 // thread.  Of whole pairs: 12 grains of up to 530 points 3.57 -> 1.83 ms, 400 of
 // 1,260-2,820 (8-bit frames of 2048x1536) 20.5 -> 7.6 ms, 2000 of up to 5,025
-// (5616x3744) 47.7 -> 26.5 ms of which the search takes 9.2.
+// (5616x3744) 47.7 -> 26.5 ms, of which the search took 9.2 then.
 template <int NT, int BLOCKS, class Ref>
 __global__ void __launch_bounds__(NT, BLOCKS) k_subpix_powell(GrainsDev g, FrameDev cur, SubpixParams sp,
                                                               int patch_cap, int max_points, const int* order,
