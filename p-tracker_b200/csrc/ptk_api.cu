@@ -372,6 +372,11 @@ int upload_patterns(ptk_ctx* c) {
   c->max_P = maxP;
   c->max_R = (int)std::ceil(maxnorm) + 1;
   c->powell = PowellSizes{n, maxP, c->max_R, n_large, small_P, (int)std::ceil(small_norm) + 1};
+  if (powell_split(c->powell, c->num_sms)) {  // (a context that never splits a launch is created 80 us sooner)
+    if (!c->side.stream) CK(cudaStreamCreateWithFlags(&c->side.stream, cudaStreamNonBlocking));
+    if (!c->side.fork) CK(cudaEventCreateWithFlags(&c->side.fork, cudaEventDisableTiming));
+    if (!c->side.join) CK(cudaEventCreateWithFlags(&c->side.join, cudaEventDisableTiming));
+  }
   int max_dup = 1;
   for (int i = 0; i < n; ++i) {
     std::vector<int> keys;
@@ -844,9 +849,6 @@ int ptk_create(ptk_ctx** out, const ptk_config* cfg) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->buf_free[p], cudaEventDisableTiming);
   }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->main_mark, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side.stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->side.fork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->side.join, cudaEventDisableTiming);
   if (e != cudaSuccess) return bail(cuda_fail(c, e, "cudaEventCreate"));
   c->stream = c->own_stream;
   // rows of whole 16-byte units as they are (host rows and device rows then
