@@ -598,12 +598,13 @@ int enqueue_search(ptk_ctx* c, int level, cudaStream_t s, cudaEvent_t* ev = null
   if ((sg.bf16 && (c->bf_cap < sg.items || c->bf_geom_dirty)) || c->best_cap < sx.items)
     return fail(c, PTK_ERR_STATE, "search scratch not prepared");
   if (level == 0) {
-    launch_stage_begin(c->g, c->d_counts, s);
+    launch_stage_begin(c->g, c->d_counts, c->d_work, s);
     c->launches += 1;
+  } else {
+    CK(cudaMemsetAsync(c->d_work, 0, 2 * sizeof(int), s));
   }
   const int* list = level == 0 ? c->d_order : (level == 1 ? c->d_lists : c->d_lists + c->n);
   const int* count = c->d_counts + level;
-  CK(cudaMemsetAsync(c->d_work, 0, 2 * sizeof(int), s));
   const ptk_zone& z = c->cfg.zone[level];
   FinalizeLaunch f;
   f.g = c->g;
@@ -722,7 +723,7 @@ int enqueue_subpixel(ptk_ctx* c, int method, cudaStream_t s) {
                       ? c->cfg.lm_cell_rot * z0.inc_rot
                       : HUGE_VAL;
     if (!(lp.cell_px > 0.0)) lp.redo_list = nullptr;  // hand-off disabled: every LM result is kept
-    CK(cudaMemsetAsync(lp.redo_count, 0, sizeof(int), s));
+    if (lp.redo_list) CK(cudaMemsetAsync(lp.redo_count, 0, sizeof(int), s));
     launch_subpix_lm(c->g, frame(c, c->cur_slot), lp, s);
     if (lp.redo_list) {  // those grains: the reference's Powell from their pixel-stage state
       launch_subpix_powell(c->g, frame(c, c->cur_slot), subpix_params(c), c->powell, c->num_sms, lp.redo_list, s,

@@ -164,7 +164,7 @@ void launch_subpix_lm(const GrainsDev& g, const FrameDev& cur, const LmParams& l
 void launch_grad_f32(const GrainsDev& g, const FrameDev& cur, const double* X, double* f, double* grad,
                      cudaStream_t s);
 void launch_precompute(const GrainsDev& g, const FrameDev& ref, cudaStream_t s);
-void launch_stage_begin(const GrainsDev& g, int* counts, cudaStream_t s);
+void launch_stage_begin(const GrainsDev& g, int* counts, int* work, cudaStream_t s);
 void launch_search(const SearchLaunch& p, int grid, size_t smem, cudaStream_t s);
 size_t search_smem_bytes(int max_points, int max_patch_elems);
 int search_occupancy(size_t smem);

@@ -109,12 +109,13 @@ __global__ void k_precompute(GrainsDev g, FrameDev ref) {
 
 // reset() + backup() of every grain at the start of the pixel stage
 // (src/p-tracker.cpp:478-479) and zeroing of the list counters.
-__global__ void k_stage_begin(GrainsDev g, int* counts) {
+__global__ void k_stage_begin(GrainsDev g, int* counts, int* work) {
   const int gi = blockIdx.x * blockDim.x + threadIdx.x;
   if (gi == 0) {
     counts[1] = 0;
     counts[2] = 0;
     counts[4] = counts[5] = counts[6] = 0;  // exact re-search lists of BF16 levels
+    work[0] = work[1] = 0;                  // work queues of the level's search kernels
   }
   if (gi >= g.n) return;
   g.ncc[gi] = 0.0;
@@ -457,9 +458,9 @@ void launch_precompute(const GrainsDev& g, const FrameDev& ref, cudaStream_t s) 
   if (g.n > 0) k_precompute<<<g.n, 256, 0, s>>>(g, ref);
 }
 
-void launch_stage_begin(const GrainsDev& g, int* counts, cudaStream_t s) {
+void launch_stage_begin(const GrainsDev& g, int* counts, int* work, cudaStream_t s) {
   const int n = g.n > 0 ? g.n : 1;
-  k_stage_begin<<<(n + 255) / 256, 256, 0, s>>>(g, counts);
+  k_stage_begin<<<(n + 255) / 256, 256, 0, s>>>(g, counts, work);
 }
 
 static void search_attr(size_t smem) { ensure_smem((const void*)k_search, smem); }
