@@ -1048,13 +1048,15 @@ int ptk_get_grains(ptk_ctx* c, ptk_grain* out, int n) {
   if (n != c->n) return fail(c, PTK_ERR_ARG, "grain count mismatch");
   if (n == 0) return PTK_OK;
   BlockLayout L(n);
-  CK(cudaStreamSynchronize(c->stream));
-  all_released(c);
+  // the copy follows the frame's kernels (and an upload from the staging buffer)
+  // on the stream; one wait for all of it
+  if (L.total > c->h_stage_bytes) CK(cudaStreamSynchronize(c->stream));  // (the buffer is replaced)
   int rc = ensure_stage(c, L.total);
   if (rc) return rc;
   const char* h = static_cast<const char*>(c->h_stage);
   CK(cudaMemcpyAsync(c->h_stage, c->d_block, L.total, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  all_released(c);
   const size_t nn = (size_t)n;
   auto D = [&](int k) { return reinterpret_cast<const double*>(h + L.d_off + k * nn * 8); };
   auto I = [&](int k) { return reinterpret_cast<const int*>(h + L.i_off + k * nn * 4); };
