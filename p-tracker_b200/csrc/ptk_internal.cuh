@@ -174,7 +174,12 @@ void launch_search_tiled(const SearchLaunch& p, int max_r, int grid, size_t smem
 void launch_finalize(const FinalizeLaunch& p, int n_grains, cudaStream_t s);
 bool bf16_supported(int max_r, int nrot, int max_dup);
 bool bf16_ring_ok(int max_half, int ring);
-constexpr int kBf16RingDefault = 4;
+// operand-row buffers of the search kernel: three leave taller strips of image
+// rows than four (whole pairs, precision form: 2000 grains +-15 1225 -> 1205 us,
+// 5000 grains in two frames with rescues 8.77 -> 8.71 ms; 400 grains +-8 474 ->
+// 475, 40 grains 162 -> 161 us); two and six are slower (1.07 and 1.33 ms against
+// 1.01 for the search's three kernels at 2000 grains)
+constexpr int kBf16RingDefault = 3;
 size_t bf16_weight_entries(int half);
 int bf16_weight_splits(int n, int nrot, int num_sms);
 bool bf16_encode_tmaps(const int* half, const size_t* wofs, int n, unsigned char* wslots, int nrot,
