@@ -311,7 +311,7 @@ int ptk_save_grains_file(const char* path, const ptk_grain* grains, int n, const
  * warm-up), each after a 256 MiB write that evicts L2 (when that much memory
  * is free), from the same grain state (restored after every run and at the
  * end), and keeps the fastest for this context until its search method or
- * level-0 zone changes; the built-in shape (4 buffers, the tiled kernel)
+ * level-0 zone changes; the built-in shape (3 buffers, the tiled kernel)
  * stays unless another is more than 2 % faster.  Every candidate gives the same results.  With
  * ptk_config.autotune = 1, ptk_track_frame calls it once before building its
  * first graph.  report (may be NULL): method 1 = BF16 (values = ring depths),

@@ -113,7 +113,7 @@ constexpr long kDrainLimit = 1L << 26;
 constexpr int kRowThread = 32;  // issues the operand rows' copies during the MMA phases
 constexpr int kNextWarp = 2;    // fetches the next work item during a tile's first MMA phase
 constexpr int kRing = 8;       // barrier slots
-constexpr int kRingUsed = 4;   // buffers
+constexpr int kRingUsed = 4;   // buffers that every admitted geometry has room for (the default uses 3)
 // weights kernel: 512 threads, 108 KB of 32-bit maps (two blocks per SM, as
 // its registers allow)
 constexpr int kWThreads = 512;
